@@ -193,4 +193,23 @@ __device__ __forceinline__ int64_t first_row_at(const int64_t* __restrict__ ptr,
   return lo;
 }
 
+// The same by a whole warp: 32 probes a round, so 4 dependent loads for a
+// million rows instead of 20.  Every lane gets the answer.
+__device__ __forceinline__ int64_t warp_first_row_at(const int64_t* __restrict__ ptr, int64_t rows,
+                                                     int64_t weight, int64_t target, int lane) {
+  int64_t lo = 0;
+  int64_t hi = rows;
+  while (lo < hi) {
+    const int64_t len = hi - lo;
+    const bool last = len <= 32;
+    const int64_t at = last ? lo + lane : lo + len * lane / 32;
+    const bool below = at < hi && weight * at + __ldg(ptr + at) < target;
+    const int n = __popc(__ballot_sync(0xffffffffu, below));  // the probes are increasing
+    if (last || n == 0) return lo + n;
+    if (n < 32) hi = lo + len * n / 32;
+    lo = lo + len * (n - 1) / 32 + 1;
+  }
+  return lo;
+}
+
 }  // namespace ascb

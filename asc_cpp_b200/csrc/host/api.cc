@@ -464,7 +464,7 @@ PlanLayout PlanLayoutFor(const asc_sb_sparse& m, int flags) {
     l.t_part = at;
     at += PartitionBytes(inner, nnz);
     l.sort = at;
-    at += RoundUp(ascb_sort_workspace_bytes(nnz, inner), 256);
+    at += RoundUp(ascb_sort_workspace_bytes(nnz, inner, outer, 0), 256);
     l.outer_of = at;
     at += EntryBytes(nnz, 8);
   }
@@ -552,22 +552,24 @@ Status BuildStaged(asc_sb_context* ctx, asc_sb_plan* plan) {
 }
 
 // Stable transposed structure of the CSR arrays `a` (rows = stored outer
-// extent): t_ptr [a.cols + 1], t_idx / t_perm / t_val [nnz].
+// extent): t_ptr [a.cols + 1], t_idx / t_val [nnz], and t_perm [nnz] unless it
+// is null.
 Status BuildTransposed(asc_sb_context* ctx, const ascb_csr& a, std::size_t element,
                        std::int64_t* t_ptr, std::int64_t* t_idx, std::int64_t* t_perm,
                        void* t_val, void* sort_scratch, std::int64_t* outer_of) {
-  Status s = Launched(ctx,
-                      ascb_stable_sort(ctx->stream, a.idx, 1, a.nnz, a.cols, t_ptr, t_perm,
-                                       sort_scratch),
-                      "CUDA could not launch the transposition sort");
-  if (!s.ok()) return s;
-  s = Launched(ctx, ascb_outer_of_entries(ctx->stream, a.ptr, a.rows, outer_of, ctx->sm_count),
-               "CUDA could not launch the row expansion kernel");
-  if (!s.ok()) return s;
+  ascb_sort_emit emit{};
+  emit.ptr = a.ptr;
+  emit.outer = a.rows;
+  emit.outer_of = outer_of;
+  emit.other_limit = a.rows;
+  emit.idx_out = t_idx;
+  emit.val_in = a.val;
+  emit.val_out = t_val;
+  emit.elem_bytes = static_cast<int>(element);
   return Launched(ctx,
-                  ascb_permute_entries(ctx->stream, t_perm, a.nnz, outer_of, 1, t_idx, a.val,
-                                       t_val, static_cast<int>(element), ctx->sm_count),
-                  "CUDA could not launch the entry permutation kernel");
+                  ascb_stable_sort(ctx->stream, a.idx, 1, a.nnz, a.cols, t_ptr, t_perm,
+                                   sort_scratch, &emit),
+                  "CUDA could not launch the transposition sort");
 }
 
 // ---- variant selector ------------------------------------------------------
@@ -1077,12 +1079,10 @@ Status TransposedInScratch(asc_sb_context* ctx, const ascb_csr& a, std::size_t e
   total += RoundUp(static_cast<std::size_t>(a.cols + 1) * 8, 256);
   const std::size_t t_idx = total;
   total += EntryBytes(nnz, 8);
-  const std::size_t t_perm = total;
-  total += EntryBytes(nnz, 8);
   const std::size_t t_val = total;
   total += EntryBytes(nnz, element);
   const std::size_t sort = total;
-  total += RoundUp(ascb_sort_workspace_bytes(nnz, a.cols), 256);
+  total += RoundUp(ascb_sort_workspace_bytes(nnz, a.cols, a.rows, static_cast<int>(element)), 256);
   const std::size_t outer_of = total;
   total += EntryBytes(nnz, 8);
   unsigned char* base = nullptr;
@@ -1090,8 +1090,8 @@ Status TransposedInScratch(asc_sb_context* ctx, const ascb_csr& a, std::size_t e
   if (!s.ok()) return s;
   auto* tp = reinterpret_cast<std::int64_t*>(base + t_ptr);
   auto* ti = reinterpret_cast<std::int64_t*>(base + t_idx);
-  s = BuildTransposed(ctx, a, element, tp, ti, reinterpret_cast<std::int64_t*>(base + t_perm),
-                      base + t_val, base + sort, reinterpret_cast<std::int64_t*>(base + outer_of));
+  s = BuildTransposed(ctx, a, element, tp, ti, nullptr, base + t_val, base + sort,
+                      reinterpret_cast<std::int64_t*>(base + outer_of));
   if (!s.ok()) return s;
   *out = ascb_csr{};
   out->rows = a.cols;
@@ -1468,9 +1468,9 @@ int asc_sb_plan_refresh_values(asc_sb_context* ctx, asc_sb_plan* plan) {
   if (!guard.ok()) return Finish(ctx, Fail(ASC_SB_UNAVAILABLE, "CUDA device is unavailable"));
   // the transposed values are a gather of the stored ones through t_perm
   return Finish(ctx, Launched(ctx,
-                              ascb_permute_entries(
-                                  ctx->stream, plan->t_perm, plan->matrix.nonzeros, nullptr, 0,
-                                  nullptr, plan->matrix.values, plan->t_val,
+                              ascb_permute_values(
+                                  ctx->stream, plan->t_perm, plan->matrix.nonzeros,
+                                  plan->matrix.values, plan->t_val,
                                   static_cast<int>(ascb::host::ElementBytes(plan->matrix.element_kind)),
                                   ctx->sm_count),
                               "CUDA could not launch the entry permutation kernel"));
@@ -1535,18 +1535,18 @@ int asc_sb_plan_standard_spmm(asc_sb_context* ctx, const asc_sb_plan* plan, int3
 namespace {
 
 struct ConvertLayout {
-  std::size_t perm = 0, outer_of = 0, sort = 0, total = 0;
+  std::size_t outer_of = 0, sort = 0, total = 0;
 };
 
-ConvertLayout ConvertLayoutFor(std::int64_t nnz, std::int64_t destination_outer) {
+// (sized for elements of 16 bytes: the workspace query has no element kind)
+ConvertLayout ConvertLayoutFor(std::int64_t nnz, std::int64_t destination_outer,
+                               std::int64_t destination_inner) {
   ConvertLayout l;
   std::size_t at = 0;
-  l.perm = at;
-  at += EntryBytes(nnz, 8);
   l.outer_of = at;
   at += EntryBytes(nnz, 8);
   l.sort = at;
-  at += RoundUp(ascb_sort_workspace_bytes(nnz, destination_outer), 256);
+  at += RoundUp(ascb_sort_workspace_bytes(nnz, destination_outer, destination_inner, 16), 256);
   l.total = at;
   return l;
 }
@@ -1600,7 +1600,8 @@ int asc_sb_convert_workspace_size(asc_sb_context* ctx, int64_t rows, int64_t col
   if (rows < 0 || columns < 0 || nonzeros < 0) {
     return Finish(ctx, Fail(ASC_SB_SHAPE, "conversion extents cannot be negative"));
   }
-  *bytes = ConvertLayoutFor(nonzeros, destination_format == ASC_SB_CSR ? rows : columns).total;
+  const bool to_csr = destination_format == ASC_SB_CSR;
+  *bytes = ConvertLayoutFor(nonzeros, to_csr ? rows : columns, to_csr ? columns : rows).total;
   return Finish(ctx, Status::Ok());
 }
 
@@ -1625,9 +1626,10 @@ int asc_sb_convert_compressed(asc_sb_context* ctx, const asc_sb_sparse* source,
     return Finish(ctx, Fail(ASC_SB_INVALID_ARGUMENT,
                             "a compressed conversion goes from CSR to CSC or from CSC to CSR"));
   }
-  const std::int64_t dest_outer =
-      destination->format == ASC_SB_CSR ? source->rows : source->columns;
-  const ConvertLayout l = ConvertLayoutFor(source->nonzeros, dest_outer);
+  const bool to_csr = destination->format == ASC_SB_CSR;
+  const ConvertLayout l =
+      ConvertLayoutFor(source->nonzeros, to_csr ? source->rows : source->columns,
+                       to_csr ? source->columns : source->rows);
   s = ValidateConvertWorkspace(ctx, workspace, workspace_bytes, l.total);
   if (!s.ok()) return Finish(ctx, s);
   const Span ws{workspace, workspace_bytes};
@@ -1645,11 +1647,10 @@ int asc_sb_convert_compressed(asc_sb_context* ctx, const asc_sb_sparse* source,
   // indices, which become the destination's outer indices
   const ascb_csr a = AsCsr(*source, source->format == ASC_SB_CSC);
   auto* w = static_cast<unsigned char*>(workspace);
-  auto* perm = reinterpret_cast<std::int64_t*>(w + l.perm);
   s = BuildTransposed(ctx, a, ascb::host::ElementBytes(source->element_kind),
                       static_cast<std::int64_t*>(const_cast<void*>(destination->structure_first)),
                       static_cast<std::int64_t*>(const_cast<void*>(destination->structure_second)),
-                      perm, const_cast<void*>(destination->values), w + l.sort,
+                      nullptr, const_cast<void*>(destination->values), w + l.sort,
                       reinterpret_cast<std::int64_t*>(w + l.outer_of));
   return Finish(ctx, s);
 }
@@ -1689,7 +1690,8 @@ int asc_sb_convert_coordinates(asc_sb_context* ctx, const int64_t* coordinates,
     if (!s.ok()) return Finish(ctx, s);
   }
   const bool to_csr = destination->format == ASC_SB_CSR;
-  const ConvertLayout l = ConvertLayoutFor(nonzeros, to_csr ? rows : columns);
+  const ConvertLayout l =
+      ConvertLayoutFor(nonzeros, to_csr ? rows : columns, to_csr ? columns : rows);
   s = ValidateConvertWorkspace(ctx, workspace, workspace_bytes, l.total);
   if (!s.ok()) return Finish(ctx, s);
   const Span ws{workspace, workspace_bytes};
@@ -1700,22 +1702,23 @@ int asc_sb_convert_coordinates(asc_sb_context* ctx, const int64_t* coordinates,
                             "conversion destination and workspace must not overlap any operand"));
   }
   auto* w = static_cast<unsigned char*>(workspace);
-  auto* perm = reinterpret_cast<std::int64_t*>(w + l.perm);
-  auto* offsets = static_cast<std::int64_t*>(const_cast<void*>(destination->structure_first));
   // coordinates are (row, column) pairs: the destination's outer index is the
   // row for CSR and the column for CSC, the other one becomes the inner index
+  ascb_sort_emit emit{};
+  emit.other = coordinates + (to_csr ? 1 : 0);
+  emit.ostride = 2;
+  emit.other_limit = to_csr ? columns : rows;
+  emit.idx_out = static_cast<std::int64_t*>(const_cast<void*>(destination->structure_second));
+  emit.val_in = values;
+  emit.val_out = const_cast<void*>(destination->values);
+  emit.elem_bytes = static_cast<int>(element);
   s = Launched(ctx,
                ascb_stable_sort(ctx->stream, coordinates + (to_csr ? 0 : 1), 2, nonzeros,
-                                to_csr ? rows : columns, offsets, perm, w + l.sort),
+                                to_csr ? rows : columns,
+                                static_cast<std::int64_t*>(
+                                    const_cast<void*>(destination->structure_first)),
+                                nullptr, w + l.sort, &emit),
                "CUDA could not launch the conversion sort");
-  if (!s.ok()) return Finish(ctx, s);
-  s = Launched(ctx,
-               ascb_permute_entries(
-                   ctx->stream, perm, nonzeros, coordinates + (to_csr ? 1 : 0), 2,
-                   static_cast<std::int64_t*>(const_cast<void*>(destination->structure_second)),
-                   values, const_cast<void*>(destination->values), static_cast<int>(element),
-                   ctx->sm_count),
-               "CUDA could not launch the entry permutation kernel");
   return Finish(ctx, s);
 }
 
@@ -1911,18 +1914,16 @@ Status TriangularSolve(asc_sb_context* ctx, const asc_sb_plan* plan, int op, dou
         RoundUp(ascb_trsv_scratch_bytes(n, static_cast<int>(element)), 256);
     const std::int64_t nnz = m->nonzeros;
     std::size_t total = flags;
-    std::size_t t_ptr = 0, t_idx = 0, t_perm = 0, t_val = 0, sort = 0, outer_of = 0;
+    std::size_t t_ptr = 0, t_idx = 0, t_val = 0, sort = 0, outer_of = 0;
     if (transposed && !alpha_zero) {
       t_ptr = total;
       total += RoundUp(static_cast<std::size_t>(n + 1) * 8, 256);
       t_idx = total;
       total += EntryBytes(nnz, 8);
-      t_perm = total;
-      total += EntryBytes(nnz, 8);
       t_val = total;
       total += EntryBytes(nnz, element);
       sort = total;
-      total += RoundUp(ascb_sort_workspace_bytes(nnz, n), 256);
+      total += RoundUp(ascb_sort_workspace_bytes(nnz, n, n, static_cast<int>(element)), 256);
       outer_of = total;
       total += EntryBytes(nnz, 8);
     }
@@ -1931,9 +1932,8 @@ Status TriangularSolve(asc_sb_context* ctx, const asc_sb_plan* plan, int op, dou
     if (transposed && !alpha_zero) {
       auto* tp = reinterpret_cast<std::int64_t*>(control + t_ptr);
       auto* ti = reinterpret_cast<std::int64_t*>(control + t_idx);
-      s = BuildTransposed(ctx, op_csr, element, tp, ti,
-                          reinterpret_cast<std::int64_t*>(control + t_perm), control + t_val,
-                          control + sort, reinterpret_cast<std::int64_t*>(control + outer_of));
+      s = BuildTransposed(ctx, op_csr, element, tp, ti, nullptr, control + t_val, control + sort,
+                          reinterpret_cast<std::int64_t*>(control + outer_of));
       if (!s.ok()) return s;
       op_csr.ptr = tp;
       op_csr.idx = ti;

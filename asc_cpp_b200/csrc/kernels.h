@@ -47,19 +47,36 @@ int ascb_merge_path_splits(void* stream, const ascb_csr* a, int64_t items,
 
 // ---- stable sort by key (format conversions, transposed structure) ----
 // perm[q] = source position of the q-th entry in (key, position) order of
-// keys[e * kstride], e < n; offsets[0..limit] = bucket starts (keys outside
-// [0, limit) are not counted).  `workspace` holds ascb_sort_workspace_bytes.
-size_t ascb_sort_workspace_bytes(int64_t n, int64_t limit);
+// keys[e * kstride], e < n (perm may be null); offsets[0..limit] = bucket
+// starts.  Keys lie in [0, limit).  With `emit` the sort also writes the
+// entries in the new order: their new inner index and their value.
+typedef struct ascb_sort_emit {
+  // new inner index of the entry that stood at p: its outer index by `ptr`
+  // (outer + 1 offsets; outer_of: scratch of 8 bytes per entry), or, without
+  // ptr (and with perm null), other[p * ostride]; below other_limit
+  const int64_t* ptr;
+  int64_t outer;
+  void* outer_of;
+  const int64_t* other;
+  int64_t ostride;
+  int64_t other_limit;
+  int64_t* idx_out;
+  const void* val_in;  // elements of elem_bytes: 4, 8 or 16
+  void* val_out;
+  int elem_bytes;
+} ascb_sort_emit;
+// `workspace` holds ascb_sort_workspace_bytes (elem_bytes: of the values, 0
+// without them or with a permutation; other_limit: 0 without `emit`).
+size_t ascb_sort_workspace_bytes(int64_t n, int64_t limit, int64_t other_limit, int elem_bytes);
 int ascb_stable_sort(void* stream, const int64_t* keys, int64_t kstride, int64_t n, int64_t limit,
-                     int64_t* offsets, int64_t* perm, void* workspace);
-// out[q] = r for every entry q in [ptr[r], ptr[r+1]).
-int ascb_outer_of_entries(void* stream, const int64_t* ptr, int64_t outer, int64_t* out,
-                          int sm_count);
-// idx_out[j] = other[perm[j] * ostride] (if idx_out), val_out[j] =
-// val_in[perm[j]] (if val_out; elem_bytes 4, 8 or 16).
-int ascb_permute_entries(void* stream, const int64_t* perm, int64_t n, const int64_t* other,
-                         int64_t ostride, int64_t* idx_out, const void* val_in, void* val_out,
-                         int elem_bytes, int sm_count);
+                     int64_t* offsets, int64_t* perm, void* workspace,
+                     const ascb_sort_emit* emit);
+// out[q] = r for every entry q in [ptr[r], ptr[r+1]); nnz = ptr[outer].
+int ascb_outer_of_entries(void* stream, const int64_t* ptr, int64_t outer, int64_t nnz,
+                          int64_t* out);
+// val_out[j] = val_in[perm[j]] (elem_bytes 4, 8 or 16).
+int ascb_permute_values(void* stream, const int64_t* perm, int64_t n, const void* val_in,
+                        void* val_out, int elem_bytes, int sm_count);
 
 // ---- SpMV variants ----
 // Warp-tiled SpMV over row tiles of ascb_warp_tile_items() weighted items with

@@ -412,7 +412,7 @@ int ascb_row_groups_build(void* stream, const ascb_csr* a, int elem_bytes, int r
   auto* flags = reinterpret_cast<int64_t*>(p + l.flags);
   auto* run_of = reinterpret_cast<int64_t*>(p + l.run_of);
   auto* sums = reinterpret_cast<int64_t*>(p + l.sums);
-  int rc = ascb_outer_of_entries(stream, a->ptr, a->rows, row_of, sm_count);
+  int rc = ascb_outer_of_entries(stream, a->ptr, a->rows, nnz, row_of);
   if (rc != 0) return rc;
   cudaError_t e = cudaMemsetAsync(out->run_mask, 0, static_cast<size_t>(nnz > 0 ? nnz : 1) * 4, s);
   if (e != cudaSuccess) return static_cast<int>(e);

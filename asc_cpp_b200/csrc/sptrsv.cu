@@ -760,7 +760,7 @@ extern "C" size_t ascb_trsv_analysis_bytes(int64_t n) {
   const size_t nn = static_cast<size_t>(n > 0 ? n : 0);
   auto up = [](size_t v) { return (v + 255) / 256 * 256; };
   // level, order, position, bucket offsets, sort workspace
-  return up(nn * 8) * 3 + up((nn + 2) * 8) + up(ascb_sort_workspace_bytes(n, n + 1));
+  return up(nn * 8) * 3 + up((nn + 2) * 8) + up(ascb_sort_workspace_bytes(n, n + 1, 0, 0));
 }
 
 extern "C" int ascb_trsv_analysis(void* stream, const ascb_trsv* t, void* workspace,
@@ -788,7 +788,7 @@ extern "C" int ascb_trsv_analysis(void* stream, const ascb_trsv* t, void* worksp
   int e = static_cast<int>(cudaGetLastError());
   if (e != 0) return e;
   // stable by row within a level: rows of one level in increasing order
-  e = ascb_stable_sort(stream, level, 1, n, n + 1, offsets, ord, sort_ws);
+  e = ascb_stable_sort(stream, level, 1, n, n + 1, offsets, ord, sort_ws, nullptr);
   if (e != 0) return e;
   invert_order<<<GridFor(n, 256, sm_count, 8), 256, 0, s>>>(ord, n, pos);
   return static_cast<int>(cudaGetLastError());

@@ -1,19 +1,32 @@
 // CSR x dense (SpMM) and the scatter (transpose) products, sm_100a.
 //
-// Row-major right-hand sides with 16-byte aligned rows take the chunked
-// kernel below (one vector load per lane per stored entry).  Otherwise, for
-// row-major right-hand sides:
-// a group of G lanes owns one output row o and the lanes split its k columns,
-// so each stored entry (o, c, v) costs one broadcast load of (c, v) and one
-// coalesced load of the row B(c, :).  Each lane adds its columns' terms in
-// stored order,
+// Row-major right-hand sides take the row kernel: G lanes share an output row and
+// own whole chunks of 16, 8 or 4 bytes of it (the widest that the columns and
+// strides allow), so a stored entry (o, c, v) costs one broadcast load of
+// (c, v) and one vector load per lane and chunk of the row B(c, :).  EXACT
+// adds the terms in stored order,
 //     C(o, j) = C(o, j) + (alpha * v) * B(c, j),
-// exactly the per-entry update of asc::Spmm (include/asc/sparse/blas.h:
-// 1736-1748), with every product and sum rounded separately -- so this kernel
-// is bit-exact against the serial reference and needs no separate
-// deterministic variant.
+// every product and sum rounded separately -- the per-entry update of
+// asc::Spmm (include/asc/sparse/blas.h:1736-1748), bit for bit; FAST sums with
+// FMA and applies alpha once.
 //
-// Other layouts fall back to one thread per output element (same arithmetic).
+// Rows far longer than the mean would each be one group's serial chain of
+// loads while the chip idles (a power-law matrix of 262,144 rows and 4.2 M
+// entries, FP32, B200: k = 50 950 us that way, 279 us with the rule below;
+// k = 8 968 and 79, k = 32 bit-exact 2240 and 211).
+// They are set aside and then taken by all groups of their block together:
+// FAST splits the entries and adds the groups' sums in a fixed order, EXACT
+// forms the products in parallel and adds them in stored order from shared
+// memory.
+//
+// Column-major right-hand sides: a lane per row, several columns at a time
+// (spmm_columns_kernel), with the same rule for long rows.  One thread per
+// output element, which this replaces, read every index and value once per
+// column: 27-point stencil on 80^3, FP64, k = 5 540 us against 137 (B200; DRAM
+// floor 43), k = 40 FP32 3560 against 529; power law, 100,000 rows, k = 5 1088
+// against 165.  Packing the columns into rows first measured within 10% on the
+// stencil and two to four times faster on the power law, but its scratch costs
+// 18 us per MB to allocate and cannot be used under stream capture.
 // Transposed products that have no transposed structure at hand scatter with
 // atomics (BACKEND_DEFAULT only; order-dependent rounding within the bound).
 #include "common.cuh"
@@ -25,230 +38,457 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kEntryUnroll = 4;
 
-// G lanes per row, J columns per lane (G*J >= k handled by an outer loop).
-template <typename T, int G, int J>
-__global__ void __launch_bounds__(kThreads)
-spmm_row_major_kernel(int64_t rows, int64_t k, const int64_t* __restrict__ ptr,
-                      const int64_t* __restrict__ idx, const T* __restrict__ val,
-                      const T* __restrict__ b, int64_t ldb, T* __restrict__ c,
-                      int64_t ldc, T alpha) {
-  constexpr int kGroups = kThreads / G;
-  const int lane = threadIdx.x % G;
-  const int64_t first = static_cast<int64_t>(blockIdx.x) * kGroups + threadIdx.x / G;
-  const int64_t step = static_cast<int64_t>(gridDim.x) * kGroups;
-  for (int64_t o = first; o < rows; o += step) {
-    const int64_t pb = __ldg(ptr + o);
-    const int64_t pe = __ldg(ptr + o + 1);
-    for (int64_t j0 = 0; j0 < k; j0 += int64_t{G} * J) {
-      T acc[J];
-      bool live[J];
-#pragma unroll
-      for (int t = 0; t < J; ++t) {
-        const int64_t j = j0 + t * G + lane;
-        live[t] = j < k;
-        acc[t] = live[t] ? c[o * ldc + j] : T(0);
-      }
-      int64_t q = pb;
-      for (; q + kEntryUnroll <= pe; q += kEntryUnroll) {
-        int64_t col[kEntryUnroll];
-        T av[kEntryUnroll];
-#pragma unroll
-        for (int u = 0; u < kEntryUnroll; ++u) {
-          col[u] = __ldg(idx + q + u);
-          av[u] = mul_rn(alpha, __ldg(val + q + u));
-        }
-        T bv[kEntryUnroll][J];
-#pragma unroll
-        for (int u = 0; u < kEntryUnroll; ++u) {
-#pragma unroll
-          for (int t = 0; t < J; ++t) {
-            const int64_t j = j0 + t * G + lane;
-            bv[u][t] = live[t] ? ld_gather(b + col[u] * ldb + j) : T(0);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kEntryUnroll; ++u) {
-#pragma unroll
-          for (int t = 0; t < J; ++t) acc[t] = add_rn(acc[t], mul_rn(av[u], bv[u][t]));
-        }
-      }
-      for (; q < pe; ++q) {
-        const int64_t cq = __ldg(idx + q);
-        const T av = mul_rn(alpha, __ldg(val + q));
-#pragma unroll
-        for (int t = 0; t < J; ++t) {
-          const int64_t j = j0 + t * G + lane;
-          const T bv = live[t] ? ld_gather(b + cq * ldb + j) : T(0);
-          acc[t] = add_rn(acc[t], mul_rn(av, bv));
-        }
-      }
-#pragma unroll
-      for (int t = 0; t < J; ++t) {
-        const int64_t j = j0 + t * G + lane;
-        if (live[t]) c[o * ldc + j] = acc[t];
-      }
-    }
-  }
-}
-
-// Row-major B and C with 16-byte aligned rows: each lane owns whole 16-byte
-// chunks (4 floats or 2 doubles) of the output row, so one vector load brings
-// a chunk of B(c, :) and the arithmetic per column is one multiply-add
-// (FAST) or one rounded multiply and one rounded add (EXACT, the reference's
-// per-entry update, bit-exact).  G lanes share a row; J chunks per lane.
-template <typename T>
+// N elements that are loaded at once: 16, 8 or 4 bytes.
+template <typename T, int N>
 struct Chunk;
+template <typename T>
+struct Chunk<T, 1> {
+  using type = T;
+  __device__ static void split(T v, T (&e)[1]) { e[0] = v; }
+  __device__ static T join(const T (&e)[1]) { return e[0]; }
+};
 template <>
-struct Chunk<float> {
+struct Chunk<float, 2> {
+  using type = float2;
+  __device__ static void split(const float2& v, float (&e)[2]) {
+    e[0] = v.x; e[1] = v.y;
+  }
+  __device__ static float2 join(const float (&e)[2]) { return make_float2(e[0], e[1]); }
+};
+template <>
+struct Chunk<float, 4> {
   using type = float4;
-  static constexpr int n = 4;
   __device__ static void split(const float4& v, float (&e)[4]) {
     e[0] = v.x; e[1] = v.y; e[2] = v.z; e[3] = v.w;
   }
   __device__ static float4 join(const float (&e)[4]) { return make_float4(e[0], e[1], e[2], e[3]); }
 };
 template <>
-struct Chunk<double> {
+struct Chunk<double, 2> {
   using type = double2;
-  static constexpr int n = 2;
   __device__ static void split(const double2& v, double (&e)[2]) {
     e[0] = v.x; e[1] = v.y;
   }
   __device__ static double2 join(const double (&e)[2]) { return make_double2(e[0], e[1]); }
 };
 
-template <typename T, int G, int J, bool EXACT>
-__global__ void __launch_bounds__(kThreads)
-spmm_chunk_kernel(int64_t rows, int64_t chunks, const int64_t* __restrict__ ptr,
-                  const int64_t* __restrict__ idx, const T* __restrict__ val,
-                  const T* __restrict__ b, int64_t ldb, T* __restrict__ c, int64_t ldc,
-                  T alpha) {
-  using C = Chunk<T>;
+// One product C += alpha * A * B over contiguous rows of B.
+template <typename T>
+struct RowArgs {
+  int64_t rows;
+  int64_t k;       // columns of C; the last chunk of a packed B row may pass it
+  int64_t chunks;  // chunks of a row of B
+  const int64_t* ptr;
+  const int64_t* idx;
+  const T* val;
+  const T* b;
+  int64_t ldb;    // B(c, j) = b[c * ldb + j], or b[c + j * ldb] (COLUMNS)
+  T* c;
+  int64_t c_row, c_col;  // C(o, j) = c[o * c_row + j * c_col]
+  T alpha;
+  int64_t long_row;  // rows with more entries are set aside
+};
+
+constexpr int kLongRows = 64;  // rows a block can set aside (more: taken where they stand)
+
+// Shared memory comes out of L1, which serves B to neighbouring rows (10 KB a
+// block cost the 27-point stencil 9% at k = 128), so long rows get little of
+// it.  Entries per group and round of a long row, EXACT: a round of products
+// fits 4 KB where it can.
+template <typename T, int N, int G, int J>
+__host__ __device__ constexpr int round_entries() {
+  return 4096 / (kThreads * J * N * static_cast<int>(sizeof(T))) > 0
+             ? 4096 / (kThreads * J * N * static_cast<int>(sizeof(T)))
+             : 1;
+}
+// Shared memory for a long row: a round of products, or one sum per column.
+template <typename T, int N, int G, int J, bool EXACT>
+__host__ __device__ constexpr int long_bytes() {
+  return EXACT ? kThreads * J * N * static_cast<int>(sizeof(T)) * round_entries<T, N, G, J>()
+               : G * J * N * static_cast<int>(sizeof(T));
+}
+
+// Chunk t of B's row `col`; bl: the lane's first chunk of row 0.
+template <int N, int G, bool COLUMNS, typename T>
+__device__ __forceinline__ const T* chunk_at(const RowArgs<T>& a, const T* bl, int64_t col, int t) {
+  return COLUMNS ? bl + col + t * G * a.ldb : bl + col * a.ldb + t * G * N;
+}
+
+// Entries [q, qe) of a row into acc (J chunks of N columns per lane).
+template <typename T, int N, int G, int J, bool EXACT, bool COLUMNS = false>
+__device__ __forceinline__ void add_entries(T (&acc)[J][N], const bool (&live)[J], int64_t q,
+                                            int64_t qe, const RowArgs<T>& a, const T* bl) {
+  using C = Chunk<T, N>;
   using V = typename C::type;
-  constexpr int N = C::n;
+  for (; q + kEntryUnroll <= qe; q += kEntryUnroll) {
+    int64_t col[kEntryUnroll];
+    T av[kEntryUnroll];
+#pragma unroll
+    for (int u = 0; u < kEntryUnroll; ++u) {
+      col[u] = __ldg(a.idx + q + u);
+      av[u] = EXACT ? mul_rn(a.alpha, __ldg(a.val + q + u)) : __ldg(a.val + q + u);
+    }
+    V bv[kEntryUnroll][J];
+#pragma unroll
+    for (int u = 0; u < kEntryUnroll; ++u) {
+#pragma unroll
+      for (int t = 0; t < J; ++t) {
+        bv[u][t] = live[t] ? __ldg(reinterpret_cast<const V*>(chunk_at<N, G, COLUMNS>(a, bl, col[u], t)))
+                           : V{};
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kEntryUnroll; ++u) {
+#pragma unroll
+      for (int t = 0; t < J; ++t) {
+        T e[N];
+        C::split(bv[u][t], e);
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          acc[t][i] = EXACT ? add_rn(acc[t][i], mul_rn(av[u], e[i])) : fma(av[u], e[i], acc[t][i]);
+        }
+      }
+    }
+  }
+  for (; q < qe; ++q) {
+    const int64_t cq = __ldg(a.idx + q);
+    const T av = EXACT ? mul_rn(a.alpha, __ldg(a.val + q)) : __ldg(a.val + q);
+#pragma unroll
+    for (int t = 0; t < J; ++t) {
+      if (!live[t]) continue;
+      T e[N];
+      C::split(__ldg(reinterpret_cast<const V*>(chunk_at<N, G, COLUMNS>(a, bl, cq, t))), e);
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        acc[t][i] = EXACT ? add_rn(acc[t][i], mul_rn(av, e[i])) : fma(av, e[i], acc[t][i]);
+      }
+    }
+  }
+}
+
+// WHOLE: a chunk of C is one aligned vector; otherwise element by element.
+template <typename T, int N, bool WHOLE>
+__device__ __forceinline__ void load_c(const RowArgs<T>& a, int64_t o, int64_t jv, T (&e)[N]) {
+  using C = Chunk<T, N>;
+  if constexpr (WHOLE) {
+    C::split(*reinterpret_cast<const typename C::type*>(a.c + o * a.c_row + jv * N), e);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int64_t j = jv * N + i;
+      e[i] = j < a.k ? a.c[o * a.c_row + j * a.c_col] : T(0);
+    }
+  }
+}
+template <typename T, int N, bool WHOLE>
+__device__ __forceinline__ void store_c(const RowArgs<T>& a, int64_t o, int64_t jv,
+                                        const T (&e)[N]) {
+  using C = Chunk<T, N>;
+  if constexpr (WHOLE) {
+    *reinterpret_cast<typename C::type*>(a.c + o * a.c_row + jv * N) = C::join(e);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int64_t j = jv * N + i;
+      if (j < a.k) a.c[o * a.c_row + j * a.c_col] = e[i];
+    }
+  }
+}
+
+// A row set aside, by the whole block, contracted: every group sums a share
+// of the entries, shuffles join the groups of a warp, and the warps add to one
+// sum in shared memory in turn.
+template <typename T, int N, int G, int J, bool WHOLE, bool COLUMNS = false>
+__device__ __forceinline__ void long_row_fast(const RowArgs<T>& a, int64_t o, int64_t pb,
+                                              int64_t pe, T* smem) {
   constexpr int kGroups = kThreads / G;
+  const int lane = threadIdx.x % G;
+  const int group = threadIdx.x / G;
+  const int64_t share = (pe - pb + kGroups - 1) / kGroups;
+  const int64_t q0 = pb + group * share < pe ? pb + group * share : pe;
+  const int64_t q1 = q0 + share < pe ? q0 + share : pe;
+  for (int64_t v0 = 0; v0 < a.chunks; v0 += int64_t{G} * J) {
+    T acc[J][N];
+    bool live[J];
+#pragma unroll
+    for (int t = 0; t < J; ++t) {
+      live[t] = v0 + t * G + lane < a.chunks;
+#pragma unroll
+      for (int e = 0; e < N; ++e) acc[t][e] = T(0);
+    }
+    add_entries<T, N, G, J, false, COLUMNS>(acc, live, q0, q1, a,
+                                            a.b + (v0 + lane) * (COLUMNS ? a.ldb : N));
+#pragma unroll
+    for (int t = 0; t < J; ++t) {
+#pragma unroll
+      for (int e = 0; e < N; ++e) {
+#pragma unroll
+        for (int m = G; m < 32; m <<= 1) acc[t][e] += shfl_xor(acc[t][e], m);
+      }
+    }
+    for (int w = 0; w < kThreads / 32; ++w) {
+      if (static_cast<int>(threadIdx.x) / 32 == w && threadIdx.x % 32 < G) {
+#pragma unroll
+        for (int t = 0; t < J; ++t) {
+#pragma unroll
+          for (int e = 0; e < N; ++e) {
+            T& sum = smem[(t * G + lane) * N + e];
+            sum = w == 0 ? acc[t][e] : sum + acc[t][e];
+          }
+        }
+      }
+      __syncthreads();
+    }
+    if (threadIdx.x < G) {
+#pragma unroll
+      for (int t = 0; t < J; ++t) {
+        if (!live[t]) continue;
+        T sum[N], old[N];
+        load_c<T, N, WHOLE>(a, o, v0 + t * G + lane, old);
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+          sum[e] = fma(a.alpha, smem[(t * G + lane) * N + e], old[e]);
+        }
+        store_c<T, N, WHOLE>(a, o, v0 + t * G + lane, sum);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// The same in stored order: the groups form a round of products, one thread
+// per column adds them while the next round's operands are on their way.
+template <typename T, int N, int G, int J, bool COLUMNS = false>
+__device__ __forceinline__ void long_row_exact(const RowArgs<T>& a, int64_t o, int64_t pb,
+                                               int64_t pe, T* smem) {
+  using C = Chunk<T, N>;
+  using V = typename C::type;
+  constexpr int kGroups = kThreads / G;
+  constexpr int kWidth = G * J * N;  // columns of a pass
+  constexpr int kPer = round_entries<T, N, G, J>();
+  static_assert(kWidth <= kThreads, "a thread per column");
+  constexpr int kRound = kGroups * kPer;  // entries
+  const int lane = threadIdx.x % G;
+  const int group = threadIdx.x / G;
+  for (int64_t v0 = 0; v0 < a.chunks; v0 += int64_t{G} * J) {
+    const T* bl = a.b + (v0 + lane) * (COLUMNS ? a.ldb : N);
+    const int64_t j = v0 * N + threadIdx.x;  // this thread's column in the sums
+    const bool mine = static_cast<int>(threadIdx.x) < kWidth && j < a.k;
+    T sum = mine ? a.c[o * a.c_row + j * a.c_col] : T(0);
+    V bv[kPer][J];
+    T av[kPer];
+    auto fetch = [&](int64_t base) {
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        const int64_t q = base + group * kPer + u;
+        const bool ok = q < pe;
+        av[u] = ok ? mul_rn(a.alpha, __ldg(a.val + q)) : T(0);
+        const int64_t col = ok ? __ldg(a.idx + q) : 0;
+#pragma unroll
+        for (int t = 0; t < J; ++t) {
+          bv[u][t] = ok && v0 + t * G + lane < a.chunks
+                         ? __ldg(reinterpret_cast<const V*>(chunk_at<N, G, COLUMNS>(a, bl, col, t)))
+                         : V{};
+        }
+      }
+    };
+    fetch(pb);
+    for (int64_t base = pb; base < pe; base += kRound) {
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+#pragma unroll
+        for (int t = 0; t < J; ++t) {
+          T e[N];
+          C::split(bv[u][t], e);
+#pragma unroll
+          for (int i = 0; i < N; ++i) e[i] = mul_rn(av[u], e[i]);
+          *reinterpret_cast<V*>(smem + (group * kPer + u) * kWidth + (t * G + lane) * N) =
+              C::join(e);
+        }
+      }
+      __syncthreads();
+      if (base + kRound < pe) fetch(base + kRound);
+      if (mine) {
+        const int n = static_cast<int>(pe - base < kRound ? pe - base : kRound);
+#pragma unroll 8
+        for (int e = 0; e < n; ++e) sum = add_rn(sum, smem[e * kWidth + threadIdx.x]);
+      }
+      __syncthreads();
+    }
+    if (mine) a.c[o * a.c_row + j * a.c_col] = sum;
+  }
+}
+
+template <typename T, int N, int G, int J, bool EXACT, bool WHOLE>
+__global__ void __launch_bounds__(kThreads, J * N * sizeof(T) > 16 ? 4 : 5) spmm_rows_kernel(RowArgs<T> a) {
+  constexpr int kGroups = kThreads / G;
+  __shared__ __align__(16) unsigned char buffer[long_bytes<T, N, G, J, EXACT>()];
+  __shared__ int long_rows[kLongRows];  // (round, group) they came up in
+  __shared__ int long_count;
   const int lane = threadIdx.x % G;
   const int64_t first = static_cast<int64_t>(blockIdx.x) * kGroups + threadIdx.x / G;
   const int64_t step = static_cast<int64_t>(gridDim.x) * kGroups;
-  for (int64_t o = first; o < rows; o += step) {
-    const int64_t pb = __ldg(ptr + o);
-    const int64_t pe = __ldg(ptr + o + 1);
-    if (!EXACT && pb == pe) continue;
-    T* crow = c + o * ldc;
-    for (int64_t v0 = 0; v0 < chunks; v0 += int64_t{G} * J) {
-      T acc[J][N];
+  if (threadIdx.x == 0) long_count = 0;
+  __syncthreads();
+  for (int64_t o = first; o < a.rows; o += step) {
+    const int64_t pb = __ldg(a.ptr + o);
+    const int64_t pe = __ldg(a.ptr + o + 1);
+    if (pb == pe) continue;  // C keeps its bits
+    if (pe - pb > a.long_row) {
+      int at = 0;
+      if (lane == 0) at = atomicAdd(&long_count, 1);
+      if constexpr (G > 1) {
+        const unsigned group = (G == 32 ? 0xffffffffu : ((1u << (G % 32)) - 1u))
+                               << (threadIdx.x % 32 / G * G);
+        at = __shfl_sync(group, at, 0, G);
+      }
+      if (at < kLongRows) {
+        if (lane == 0) long_rows[at] = static_cast<int>((o - first) / step * kGroups + threadIdx.x / G);
+        continue;
+      }
+    }
+    for (int64_t v0 = 0; v0 < a.chunks; v0 += int64_t{G} * J) {
+      // C is read first where that costs few registers: one wait less at the end
+      constexpr bool kEarlyC = !EXACT && J * N * sizeof(T) <= 16;
+      T acc[J][N], old[J][N];
       bool live[J];
 #pragma unroll
       for (int t = 0; t < J; ++t) {
-        const int64_t jv = v0 + t * G + lane;
-        live[t] = jv < chunks;
+        live[t] = v0 + t * G + lane < a.chunks;
         if (EXACT && live[t]) {
-          C::split(*reinterpret_cast<const V*>(crow + jv * N), acc[t]);
+          load_c<T, N, WHOLE>(a, o, v0 + t * G + lane, acc[t]);
         } else {
 #pragma unroll
           for (int e = 0; e < N; ++e) acc[t][e] = T(0);
         }
+        if (kEarlyC && live[t]) load_c<T, N, WHOLE>(a, o, v0 + t * G + lane, old[t]);
       }
-      int64_t q = pb;
-      for (; q + kEntryUnroll <= pe; q += kEntryUnroll) {
-        int64_t col[kEntryUnroll];
-        T av[kEntryUnroll];
+      add_entries<T, N, G, J, EXACT>(acc, live, pb, pe, a, a.b + (v0 + lane) * N);
 #pragma unroll
-        for (int u = 0; u < kEntryUnroll; ++u) {
-          col[u] = __ldg(idx + q + u);
-          av[u] = EXACT ? mul_rn(alpha, __ldg(val + q + u)) : __ldg(val + q + u);
+      for (int t = 0; t < J; ++t) {
+        if (!live[t]) continue;
+        if (!EXACT) {
+          if (!kEarlyC) load_c<T, N, WHOLE>(a, o, v0 + t * G + lane, old[t]);
+#pragma unroll
+          for (int i = 0; i < N; ++i) acc[t][i] = fma(a.alpha, acc[t][i], old[t][i]);
         }
-        V bv[kEntryUnroll][J];
+        store_c<T, N, WHOLE>(a, o, v0 + t * G + lane, acc[t]);
+      }
+    }
+  }
+  __syncthreads();
+  const int count = long_count < kLongRows ? long_count : kLongRows;
+  for (int i = 0; i < count; ++i) {
+    const int64_t o = static_cast<int64_t>(blockIdx.x) * kGroups + long_rows[i] % kGroups +
+                      long_rows[i] / kGroups * step;
+    const int64_t pb = __ldg(a.ptr + o);
+    const int64_t pe = __ldg(a.ptr + o + 1);
+    if constexpr (EXACT) {
+      long_row_exact<T, N, G, J>(a, o, pb, pe, reinterpret_cast<T*>(buffer));
+    } else {
+      long_row_fast<T, N, G, J, WHOLE>(a, o, pb, pe, reinterpret_cast<T*>(buffer));
+    }
+  }
+}
+
+// Column-major right-hand sides: a lane owns a row and KC columns of it, so an
+// entry's index and value are read once for KC columns and neighbouring rows,
+// whose columns are mostly neighbours too, read neighbouring elements of B.
+// Entries come four at a time in 32-byte loads from the aligned position at or
+// before the row's first (VEC: both arrays on 32-byte boundaries); a lane has
+// 4 KC elements of B in flight.  Rows above the limit are set aside for the
+// whole block, lanes over columns.
+template <typename T, int KC, bool EXACT, bool VEC>
+__global__ void __launch_bounds__(kThreads) spmm_columns_kernel(RowArgs<T> a, int64_t nnz) {
+  __shared__ __align__(16) unsigned char buffer[long_bytes<T, 1, 8, 1, EXACT>()];
+  __shared__ int long_rows[kThreads];
+  __shared__ int long_count;
+  for (int64_t o0 = static_cast<int64_t>(blockIdx.x) * kThreads; o0 < a.rows;
+       o0 += static_cast<int64_t>(gridDim.x) * kThreads) {
+    const int64_t o = o0 + threadIdx.x;
+    const int64_t pb = o < a.rows ? __ldg(a.ptr + o) : 0;
+    const int64_t pe = o < a.rows ? __ldg(a.ptr + o + 1) : 0;
+    if (threadIdx.x == 0) long_count = 0;
+    __syncthreads();
+    const bool set_aside = pe - pb > a.long_row;
+    if (set_aside) long_rows[atomicAdd(&long_count, 1)] = static_cast<int>(threadIdx.x);
+    int count = -1;  // known once every lane has been here
+    for (int64_t j0 = int64_t{KC} * blockIdx.y; j0 < a.k; j0 += int64_t{KC} * gridDim.y) {
+      RowArgs<T> part = a;  // this pass's columns
+      part.k = a.k - j0 < KC ? a.k - j0 : KC;
+      part.chunks = part.k;
+      part.b = a.b + j0 * a.ldb;
+      part.c = a.c + j0 * a.c_col;
+      if (pb < pe && !set_aside) {
+        T acc[KC];
+        T* cp = part.c + o * a.c_row;
 #pragma unroll
-        for (int u = 0; u < kEntryUnroll; ++u) {
+        for (int u = 0; u < KC; ++u) acc[u] = EXACT && u < part.k ? cp[u * a.c_col] : T(0);
+        for (int64_t q = VEC ? pb & ~int64_t{3} : pb; q < pe; q += 4) {
+          int64_t col[4];
+          T av[4];
+          if (VEC && q + 4 <= nnz) {
+            ld_stream32(a.idx + q, col);
+            if constexpr (sizeof(T) == 8) {
+              ld_stream32(a.val + q, av);
+            } else {
+              const float4 v = __ldcs(reinterpret_cast<const float4*>(a.val + q));
+              av[0] = v.x, av[1] = v.y, av[2] = v.z, av[3] = v.w;
+            }
+          } else {
 #pragma unroll
-          for (int t = 0; t < J; ++t) {
-            const int64_t jv = v0 + t * G + lane;
-            bv[u][t] = live[t] ? __ldg(reinterpret_cast<const V*>(b + col[u] * ldb + jv * N))
-                               : V{};
+            for (int e = 0; e < 4; ++e) {
+              const bool ok = q + e >= pb && q + e < pe;
+              col[e] = ok ? __ldg(a.idx + q + e) : 0;
+              av[e] = ok ? __ldg(a.val + q + e) : T(0);
+            }
           }
-        }
+          T bv[4][KC];
 #pragma unroll
-        for (int u = 0; u < kEntryUnroll; ++u) {
+          for (int e = 0; e < 4; ++e) {
+            const bool ok = q + e >= pb && q + e < pe;
 #pragma unroll
-          for (int t = 0; t < J; ++t) {
-            T e[N];
-            C::split(bv[u][t], e);
+            for (int u = 0; u < KC; ++u) {
+              bv[e][u] = ok && u < part.k ? __ldg(part.b + col[e] + u * a.ldb) : T(0);
+            }
+          }
 #pragma unroll
-            for (int i = 0; i < N; ++i) {
-              acc[t][i] = EXACT ? add_rn(acc[t][i], mul_rn(av[u], e[i]))
-                                : fma(av[u], e[i], acc[t][i]);
+          for (int e = 0; e < 4; ++e) {
+            if (q + e < pb || q + e >= pe) continue;
+            if (EXACT) av[e] = mul_rn(a.alpha, av[e]);
+#pragma unroll
+            for (int u = 0; u < KC; ++u) {
+              acc[u] = EXACT ? add_rn(acc[u], mul_rn(av[e], bv[e][u])) : fma(av[e], bv[e][u], acc[u]);
             }
           }
         }
-      }
-      for (; q < pe; ++q) {
-        const int64_t cq = __ldg(idx + q);
-        const T av = EXACT ? mul_rn(alpha, __ldg(val + q)) : __ldg(val + q);
 #pragma unroll
-        for (int t = 0; t < J; ++t) {
-          const int64_t jv = v0 + t * G + lane;
-          if (!live[t]) continue;
-          T e[N];
-          C::split(__ldg(reinterpret_cast<const V*>(b + cq * ldb + jv * N)), e);
-#pragma unroll
-          for (int i = 0; i < N; ++i) {
-            acc[t][i] = EXACT ? add_rn(acc[t][i], mul_rn(av, e[i])) : fma(av, e[i], acc[t][i]);
-          }
+        for (int u = 0; u < KC; ++u) {
+          if (u < part.k) cp[u * a.c_col] = EXACT ? acc[u] : fma(a.alpha, acc[u], cp[u * a.c_col]);
         }
       }
-#pragma unroll
-      for (int t = 0; t < J; ++t) {
-        const int64_t jv = v0 + t * G + lane;
-        if (!live[t]) continue;
-        V* cp = reinterpret_cast<V*>(crow + jv * N);
-        if (EXACT) {
-          *cp = C::join(acc[t]);
+      if (count < 0) {
+        __syncthreads();
+        count = long_count;
+      }
+      for (int i = 0; i < count; ++i) {
+        const int64_t r = o0 + long_rows[i];
+        const int64_t rb = __ldg(a.ptr + r);
+        const int64_t re = __ldg(a.ptr + r + 1);
+        if constexpr (EXACT) {
+          long_row_exact<T, 1, 8, 1, true>(part, r, rb, re, reinterpret_cast<T*>(buffer));
         } else {
-          T old[N];
-          C::split(*cp, old);
-#pragma unroll
-          for (int i = 0; i < N; ++i) acc[t][i] = fma(alpha, acc[t][i], old[i]);
-          *cp = C::join(acc[t]);
+          long_row_fast<T, 1, 8, 1, false, true>(part, r, rb, re, reinterpret_cast<T*>(buffer));
         }
       }
     }
+    __syncthreads();  // the list is rewritten for the next rows
   }
 }
 
 __device__ __forceinline__ int64_t dense_at(int layout, int64_t ld, int64_t r,
                                             int64_t col) {
   return layout == ASCB_ROW_MAJOR ? r * ld + col : col * ld + r;
-}
-
-// Any layout: one thread per output element, entries in stored order.
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
-spmm_general_kernel(int64_t rows, int64_t k, const int64_t* __restrict__ ptr,
-                    const int64_t* __restrict__ idx, const T* __restrict__ val,
-                    const T* __restrict__ b, int b_layout, int64_t ldb,
-                    T* __restrict__ c, int c_layout, int64_t ldc, T alpha) {
-  const int64_t count = rows * k;
-  const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-       t < count; t += step) {
-    // consecutive threads take consecutive elements of C's contiguous axis
-    int64_t o, j;
-    if (c_layout == ASCB_ROW_MAJOR) {
-      o = t / k;
-      j = t % k;
-    } else {
-      j = t / rows;
-      o = t % rows;
-    }
-    T* cp = c + dense_at(c_layout, ldc, o, j);
-    T acc = *cp;
-    for (int64_t q = __ldg(ptr + o); q < __ldg(ptr + o + 1); ++q) {
-      const T av = mul_rn(alpha, __ldg(val + q));
-      acc = add_rn(acc, mul_rn(av, ld_gather(b + dense_at(b_layout, ldb, __ldg(idx + q), j))));
-    }
-    *cp = acc;
-  }
 }
 
 // Transposed product by scatter: C(c, j) += alpha * v * B(r, j) for every
@@ -281,50 +521,126 @@ unsigned grid_for(int64_t work, int per_block, int sm_count) {
   return static_cast<unsigned>(needed < resident ? (needed > 0 ? needed : 1) : resident);
 }
 
-template <typename T, int G, int J>
-int launch_rm(cudaStream_t s, const ascb_csr* a, int64_t k, const void* b,
-              int64_t ldb, void* c, int64_t ldc, T alpha, int sm) {
-  spmm_row_major_kernel<T, G, J><<<grid_for(a->rows, kThreads / G, sm), kThreads, 0, s>>>(
-      a->rows, k, a->ptr, a->idx, static_cast<const T*>(a->val),
-      static_cast<const T*>(b), ldb, static_cast<T*>(c), ldc, alpha);
-  return static_cast<int>(cudaGetLastError());
+// Rows with more entries than this are taken by a whole block: eight times the
+// mean, and at least 128 (shorter ones cost less than the block's barriers).
+int64_t long_row_limit(const ascb_csr* a) {
+  const int64_t mean = a->nnz / (a->rows > 0 ? a->rows : 1);
+  return 8 * mean > 128 ? 8 * mean : 128;
 }
 
-template <typename T, int G, int J>
-int launch_chunks(cudaStream_t s, bool exact, const ascb_csr* a, int64_t chunks, const void* b,
-                  int64_t ldb, void* c, int64_t ldc, T alpha, int sm) {
-  const unsigned grid = grid_for(a->rows, kThreads / G, sm);
-  const auto* val = static_cast<const T*>(a->val);
+template <typename T, int N, int G, int J>
+int launch_rows(cudaStream_t s, bool exact, bool whole, const RowArgs<T>& a, int sm) {
+  const unsigned grid = grid_for(a.rows, kThreads / G, sm);
   if (exact) {
-    spmm_chunk_kernel<T, G, J, true><<<grid, kThreads, 0, s>>>(
-        a->rows, chunks, a->ptr, a->idx, val, static_cast<const T*>(b), ldb,
-        static_cast<T*>(c), ldc, alpha);
+    if (whole) {
+      spmm_rows_kernel<T, N, G, J, true, true><<<grid, kThreads, 0, s>>>(a);
+    } else {
+      spmm_rows_kernel<T, N, G, J, true, false><<<grid, kThreads, 0, s>>>(a);
+    }
+  } else if (whole) {
+    spmm_rows_kernel<T, N, G, J, false, true><<<grid, kThreads, 0, s>>>(a);
   } else {
-    spmm_chunk_kernel<T, G, J, false><<<grid, kThreads, 0, s>>>(
-        a->rows, chunks, a->ptr, a->idx, val, static_cast<const T*>(b), ldb,
-        static_cast<T*>(c), ldc, alpha);
+    spmm_rows_kernel<T, N, G, J, false, false><<<grid, kThreads, 0, s>>>(a);
   }
   return static_cast<int>(cudaGetLastError());
 }
 
-// Chunked kernel choice, measured on B200 with the 27-point stencil and the
-// 16 x 16 block-sparse matrices: a row's chunks are spread over G lanes, J
+// Lanes and chunks per lane, measured on B200 with the 27-point stencil and
+// the 16 x 16 block-sparse matrices: a row's chunks are spread over G lanes, J
 // chunks per lane.  Up to two chunks per row take one lane each (more rows
 // per warp); wider rows take two chunks per lane (more independent loads in
 // flight, and a CTA covers more consecutive rows whose right-hand-side rows
-// then hit in L1).
+// then hit in L1).  Single elements: up to four per lane, so that k = 128
+// reads a row's entries once.
+template <typename T, int N>
+int launch_by_width(cudaStream_t s, bool exact, bool whole, const RowArgs<T>& a, int sm) {
+#define ASCB_ROWS(G, J) return launch_rows<T, N, G, J>(s, exact, whole, a, sm)
+  if (a.chunks <= 1) ASCB_ROWS(1, 1);
+  if (a.chunks <= 2) ASCB_ROWS(2, 1);
+  if (a.chunks <= 4) ASCB_ROWS(2, 2);
+  if (a.chunks <= 8) ASCB_ROWS(4, 2);
+  if (a.chunks <= 16) ASCB_ROWS(8, 2);
+  if constexpr (N * sizeof(T) < 16) {
+    if (a.chunks > 32) {
+      if constexpr (N == 1) {
+        if (a.chunks > 64) ASCB_ROWS(32, 4);
+      }
+      ASCB_ROWS(32, 2);
+    }
+  }
+  ASCB_ROWS(16, 2);
+#undef ASCB_ROWS
+}
+
+// B in rows of `width` >= k elements (width > k: packed, zeros past k).
 template <typename T>
-int launch_chunked(cudaStream_t s, bool exact, const ascb_csr* a, int64_t chunks,
-                   const void* b, int64_t ldb, void* c, int64_t ldc, T alpha, int sm) {
-#define ASCB_CHUNKS(G, J) \
-  return launch_chunks<T, G, J>(s, exact, a, chunks, b, ldb, c, ldc, alpha, sm)
-  if (chunks <= 1) ASCB_CHUNKS(1, 1);
-  if (chunks <= 2) ASCB_CHUNKS(2, 1);
-  if (chunks <= 4) ASCB_CHUNKS(2, 2);
-  if (chunks <= 8) ASCB_CHUNKS(4, 2);
-  if (chunks <= 16) ASCB_CHUNKS(8, 2);
-  ASCB_CHUNKS(16, 2);
-#undef ASCB_CHUNKS
+int spmm_rows(cudaStream_t s, bool exact, const ascb_csr* m, int64_t k, const void* b,
+              int64_t width, int64_t ldb, void* c, int c_layout, int64_t ldc, T alpha, int sm) {
+  constexpr int kMost = 16 / sizeof(T);
+  RowArgs<T> a{m->rows, k, 0, m->ptr, m->idx, static_cast<const T*>(m->val),
+               static_cast<const T*>(b), ldb, static_cast<T*>(c), 1, 1, alpha, long_row_limit(m)};
+  (c_layout == ASCB_ROW_MAJOR ? a.c_row : a.c_col) = ldc;
+  auto divides = [](int64_t n, int64_t w, int64_t ld, const void* p) {
+    return w % n == 0 && ld % n == 0 &&
+           (reinterpret_cast<uintptr_t>(p) & (static_cast<uintptr_t>(n) * sizeof(T) - 1)) == 0;
+  };
+  int n = kMost;
+  while (n > 1 && !divides(n, width, ldb, b)) n /= 2;
+  bool whole = c_layout == ASCB_ROW_MAJOR && divides(n, k, ldc, c);
+  // the exact form at 32 or more 16-byte chunks per row runs faster on single
+  // elements (measured on both matrices above)
+  if (exact && n == kMost && width / n >= 32) {
+    n = 1;
+    whole = c_layout == ASCB_ROW_MAJOR;
+  }
+  a.chunks = width / n;
+  if (n == 4) {
+    if constexpr (sizeof(T) == 4) return launch_by_width<T, 4>(s, exact, whole, a, sm);
+  }
+  if (n == 2) return launch_by_width<T, 2>(s, exact, whole, a, sm);
+  return launch_by_width<T, 1>(s, exact, whole, a, sm);
+}
+
+// Rows past four times the mean and 32 go to the whole block: a warp takes as
+// long as its longest row.
+int64_t long_column_limit(const ascb_csr* a) {
+  const int64_t mean = a->nnz / (a->rows > 0 ? a->rows : 1);
+  return 4 * mean > 32 ? 4 * mean : 32;
+}
+
+template <typename T, int KC>
+int launch_columns(cudaStream_t s, bool exact, const RowArgs<T>& a, int64_t nnz, int sm) {
+  // short rows straddle two or three aligned fours: single loads serve them better
+  const bool vec =
+      nnz >= 12 * a.rows &&
+      ((reinterpret_cast<uintptr_t>(a.idx) | reinterpret_cast<uintptr_t>(a.val)) & 31u) == 0;
+  // few rows: the passes over the columns spread over the grid too
+  const unsigned blocks = grid_for(a.rows, kThreads, sm);
+  const int64_t passes = (a.k + KC - 1) / KC;
+  const int64_t room = static_cast<int64_t>(sm > 0 ? sm : 148) * 16 / blocks;
+  const dim3 grid(blocks, static_cast<unsigned>(room < 1 ? 1 : (room < passes ? room : passes)));
+  auto kernel = exact ? (vec ? spmm_columns_kernel<T, KC, true, true>
+                             : spmm_columns_kernel<T, KC, true, false>)
+                      : (vec ? spmm_columns_kernel<T, KC, false, true>
+                             : spmm_columns_kernel<T, KC, false, false>);
+  kernel<<<grid, kThreads, 0, s>>>(a, nnz);
+  return static_cast<int>(cudaGetLastError());
+}
+
+template <typename T>
+int spmm_columns(cudaStream_t s, bool exact, const ascb_csr* m, int64_t k, const void* b,
+                 int64_t ldb, void* c, int c_layout, int64_t ldc, T alpha, int sm) {
+  RowArgs<T> a{m->rows, k, k, m->ptr, m->idx, static_cast<const T*>(m->val),
+               static_cast<const T*>(b), ldb, static_cast<T*>(c), 1, 1, alpha,
+               long_column_limit(m)};
+  (c_layout == ASCB_ROW_MAJOR ? a.c_row : a.c_col) = ldc;
+  // passes of about equal width, at most 4 columns: 8 a lane (120 registers)
+  // measured 10-20% slower, a block fewer warps having to hide the gathers
+  const int64_t passes = (k + 3) / 4;
+  const int64_t width = (k + passes - 1) / passes;
+  if (width <= 1) return launch_columns<T, 1>(s, exact, a, m->nnz, sm);
+  if (width <= 2) return launch_columns<T, 2>(s, exact, a, m->nnz, sm);
+  return launch_columns<T, 4>(s, exact, a, m->nnz, sm);
 }
 
 template <typename T>
@@ -339,26 +655,10 @@ int spmm_typed(cudaStream_t s, int transpose, int exact, const ascb_csr* a, int6
         ldc, alpha);
     return static_cast<int>(cudaGetLastError());
   }
-  if (b_layout == ASCB_ROW_MAJOR && c_layout == ASCB_ROW_MAJOR) {
-    constexpr int64_t N = Chunk<T>::n;
-    const bool chunked = k % N == 0 && ldb % N == 0 && ldc % N == 0 &&
-                         ((reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15u) == 0;
-    // the exact form at 32 or more chunks per row runs faster on the scalar
-    // kernel below (measured on both matrices above)
-    if (chunked && !(exact && k / N >= 32)) {
-      return launch_chunked<T>(s, exact != 0, a, k / N, b, ldb, c, ldc, alpha, sm);
-    }
-    if (k <= 8) return launch_rm<T, 8, 1>(s, a, k, b, ldb, c, ldc, alpha, sm);
-    if (k <= 16) return launch_rm<T, 16, 1>(s, a, k, b, ldb, c, ldc, alpha, sm);
-    if (k <= 32) return launch_rm<T, 32, 1>(s, a, k, b, ldb, c, ldc, alpha, sm);
-    if (k <= 64) return launch_rm<T, 32, 2>(s, a, k, b, ldb, c, ldc, alpha, sm);
-    return launch_rm<T, 32, 4>(s, a, k, b, ldb, c, ldc, alpha, sm);
+  if (b_layout == ASCB_ROW_MAJOR) {
+    return spmm_rows<T>(s, exact != 0, a, k, b, k, ldb, c, c_layout, ldc, alpha, sm);
   }
-  spmm_general_kernel<T><<<grid_for(a->rows * k, kThreads, sm), kThreads, 0, s>>>(
-      a->rows, k, a->ptr, a->idx, static_cast<const T*>(a->val),
-      static_cast<const T*>(b), b_layout, ldb, static_cast<T*>(c), c_layout,
-      ldc, alpha);
-  return static_cast<int>(cudaGetLastError());
+  return spmm_columns<T>(s, exact != 0, a, k, b, ldb, c, c_layout, ldc, alpha, sm);
 }
 
 template <typename T, int LANES>

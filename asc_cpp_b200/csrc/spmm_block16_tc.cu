@@ -9,7 +9,11 @@
 //     D (128 x 16) = sum over the block row's blocks of  B_blk^T (128 x 16) . A_blk^T
 // i.e. D[m][n] = sum_kk B[16 bc + kk][m] A_blk[n][kk] = (A B)[16 br + n][m].
 // The product of a block is one MMA of M = 128 (right-hand sides, zero-padded),
-// N = 16 (rows of the block), K = 16 (two K = 8 steps).  Both operands are
+// N = 16 (rows of the block), K = 16 (two K = 8 steps).  What an MMA this
+// narrow costs is its 128-row operand and its issue, so hi_A and lo_A stand one
+// behind the other as one operand of N = 32 and a block takes four MMAs
+// instead of six, issued under elect.sync, which leaves their operands in
+// uniform registers (figures at ascb_spmm_block16_tc).  Both operands are
 // staged in shared memory in the canonical K-major, 64-byte-swizzle layout
 // (rows of 16 values = 64 bytes; the 16-byte chunk c of row r sits at chunk
 // c ^ ((r >> 1) & 3)), written by the threads from registers: the A block's
@@ -19,7 +23,8 @@
 // Precision: FP32 inputs are split as a = hi + lo with hi = a truncated to
 // TF32 and lo = a - hi (exact), and each block contributes
 //     hi_B hi_A + hi_B lo_A + lo_B hi_A
-// (three MMAs into the same accumulator), so the result keeps close to FP32
+// (with accumulators of their own, summed in the epilogue: the small terms do
+// not meet the large one's rounding), so the result keeps close to FP32
 // accuracy: |c - c_exact| <= (n + 64) 2^-22 |alpha| sum_k |a_k b_k| + 2^-23 |c0|
 // per output, n = stored entries in the row (tests check this bound).
 //
@@ -35,7 +40,7 @@
 // issues the B tile's bulk copy (expect-tx on the stage's `full` barrier),
 // the lanes split the block's A rows (loaded before the stage wait) into
 // hi / lo and arrive; one thread issues the MMAs as stages fill (mbarriers
-// full / empty); two 16-column accumulators alternate between block rows so
+// full / empty); two sets of accumulators alternate between block rows so
 // the epilogue of one overlaps the MMAs of the next.
 // Every wait is bounded: one that runs out records 1 in *status, tells the
 // other roles to stop (a shared flag), and the CTA waits (bounded) for its own
@@ -54,7 +59,8 @@ constexpr int kThreads = kProducerThreads + 32;  // + the MMA warp
 constexpr int kStages = kProducerWarps;          // one stage per producer warp
 constexpr int kM = 128;        // right-hand sides per pass
 constexpr int kB = 16;         // block size
-constexpr int kTmemCols = 32;  // two accumulators of 16 columns
+constexpr int kAccCols = 3 * kB;  // hi hi | hi lo | lo hi
+constexpr int kTmemCols = 128;  // two sets of accumulators (a power of two)
 constexpr uint32_t kWaitLimit = 1u << 22;
 constexpr uint32_t kSuspendNs = 1000;
 
@@ -99,9 +105,10 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr) {
   return d;
 }
 
-// instruction descriptor: D F32, A/B TF32, both K-major, N = 16, M = 128
-constexpr uint32_t kIdesc = (1u << 4) | (2u << 7) | (2u << 10) | ((16u >> 3) << 17) |
-                            ((128u >> 4) << 24);
+// instruction descriptor: D F32, A/B TF32, both K-major, M = 128
+__host__ __device__ constexpr uint32_t idesc(uint32_t n) {
+  return (1u << 4) | (2u << 7) | (2u << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
+}
 
 __device__ __forceinline__ void split(float4 v, float4& hi, float4& lo) {
   const uint32_t m = 0xffffe000u;
@@ -115,13 +122,28 @@ __device__ __forceinline__ void split(float4 v, float4& hi, float4& lo) {
   lo.w = v.w - hi.w;
 }
 
+template <uint32_t N>
 __device__ __forceinline__ void mma_tf32(uint32_t tmem, uint64_t a, uint64_t b, uint32_t acc) {
+  constexpr uint32_t kIdesc = idesc(N);
   asm volatile(
       "{\n .reg .pred p;\n"
       " setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
       "l"(a), "l"(b), "r"(kIdesc), "r"(acc)
       : "memory");
+}
+
+// One lane of a converged warp.  (Under `lane == 0` the compiler cannot keep the
+// MMA operands uniform: a block's MMAs and their commit then took 515 cycles of
+// the issuing warp, 195 this way.)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n .reg .pred p;\n"
+      " elect.sync _|p, 0xffffffff;\n"
+      " selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(p));
+  return p != 0;
 }
 
 __device__ __forceinline__ void commit(uint64_t* bar) {
@@ -233,7 +255,7 @@ block16_tc_kernel(const int64_t* __restrict__ ptr, const int64_t* __restrict__ i
   Smem& s = *reinterpret_cast<Smem*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   const int t = threadIdx.x;
-  const int warp = t >> 5;
+  const int warp = __shfl_sync(0xffffffffu, t >> 5, 0);
   const int lane = t & 31;
   if (t == 0) {
     for (int i = 0; i < kStages; ++i) {
@@ -258,7 +280,7 @@ block16_tc_kernel(const int64_t* __restrict__ ptr, const int64_t* __restrict__ i
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-  const uint32_t tmem = s.tmem;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, s.tmem, 0);
   const int64_t chunks = (k + kM - 1) / kM;
   const int64_t items = block_rows * chunks;
   bool failed = false;
@@ -325,8 +347,14 @@ block16_tc_kernel(const int64_t* __restrict__ ptr, const int64_t* __restrict__ i
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      uint32_t d[16];
-      tmem_ld16(tmem + (static_cast<uint32_t>(p * 32) << 16) + a * kB, d);
+      uint32_t d[16], e[16];
+      const uint32_t at = tmem + (static_cast<uint32_t>(p * 32) << 16) + a * kAccCols;
+      tmem_ld16(at + kB, d);
+      tmem_ld16(at + 2 * kB, e);
+      float low[kB];
+#pragma unroll
+      for (int n = 0; n < kB; ++n) low[n] = __uint_as_float(d[n]) + __uint_as_float(e[n]);
+      tmem_ld16(at, d);
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
       mbar_arrive(&s.dempty[a]);
       const int64_t m = p * 32 + lane;
@@ -334,7 +362,7 @@ block16_tc_kernel(const int64_t* __restrict__ ptr, const int64_t* __restrict__ i
 #pragma unroll
         for (int n = 0; n < kB; ++n) {
           float* cp = c + (br * kB + n) * ldc + m0 + m;
-          *cp = fmaf(alpha, __uint_as_float(d[n]), *cp);
+          *cp = fmaf(alpha, __uint_as_float(d[n]) + low[n], *cp);
         }
       }
       ++itm;
@@ -358,34 +386,31 @@ block16_tc_kernel(const int64_t* __restrict__ ptr, const int64_t* __restrict__ i
           failed = true;
           break;
         }
-        if (lane == 0) {
+        if (elect_one()) {
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
           const uint32_t base = smem_u32(&s.stage[st]);
-          const uint32_t bh = base + offsetof(Stage, bt_hi);
-          const uint32_t bl = base + offsetof(Stage, bt_lo);
-          const uint32_t ah = base + offsetof(Stage, a_hi);
-          const uint32_t al = base + offsetof(Stage, a_lo);
-          const uint32_t pa[3] = {bh, bh, bl};
-          const uint32_t pb[3] = {ah, al, ah};
+          const uint64_t bh = sdesc(base + offsetof(Stage, bt_hi));
+          const uint64_t bl = sdesc(base + offsetof(Stage, bt_lo));
+          // a_lo follows a_hi: together the 32 rows of one operand
+          const uint64_t ah = sdesc(base + offsetof(Stage, a_hi));
+          const uint32_t d = tmem + a * kAccCols;
 #pragma unroll
-          for (int q = 0; q < 3; ++q) {
-#pragma unroll
-            for (int ks = 0; ks < 2; ++ks) {
-              const uint32_t acc = (j > 0 || q > 0 || ks > 0) ? 1u : 0u;
-              mma_tf32(tmem + a * kB, sdesc(pa[q] + ks * 32), sdesc(pb[q] + ks * 32), acc);
-            }
+          for (int ks = 0; ks < 2; ++ks) {
+            const uint32_t acc = (j > 0 || ks > 0) ? 1u : 0u;
+            mma_tf32<32>(d, bh + ks * 2, ah + ks * 2, acc);
+            mma_tf32<16>(d + 2 * kB, bl + ks * 2, ah + ks * 2, acc);
           }
           commit(&s.empty[st]);
         }
         __syncwarp();
       }
       if (failed) break;
-      if (lane == 0) commit(&s.dfull[a]);
+      if (elect_one()) commit(&s.dfull[a]);
       __syncwarp();
       ++itm;
     }
     // every MMA of this CTA has completed once `done` fires
-    if (lane == 0) commit(&s.done);
+    if (elect_one()) commit(&s.done);
     __syncwarp();
     if (!wait_bar(&s.done, 0u, nullptr)) failed = true;
   }
@@ -457,6 +482,13 @@ extern "C" size_t ascb_block16_tiles_bytes(int64_t cols, int64_t k) {
          ascb::kTileFloats * sizeof(float);
 }
 
+// 65,536-row matrix with 2% dense blocks, B200, k = 8 / 32 / 128: 291 / 324 /
+// 410 us (six MMAs a block issued under `lane == 0`: 398 / 430 / 451); error
+// against 64 bits 3.4e-6 (1.0e-5).  At k = 128 the bound is the 16 KB of B images
+// a block brings from L2; below, the CTAs' MMA issue.  Feeding raw B through
+// registers into tensor memory as the MMA's A operand (8 KB a block, no
+// pre-pass, 20 warps in one CTA) measured 427 / 423 / 431: each set of four
+// warps spends about 1,050 cycles of dependent work on a block.
 extern "C" int ascb_spmm_block16_tc(void* stream, const ascb_csr* a, int64_t k, const float* b,
                                     int64_t ldb, float* c, int64_t ldc, float alpha,
                                     float* tiles, int* status, int sm_count) {

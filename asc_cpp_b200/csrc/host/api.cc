@@ -1945,6 +1945,7 @@ Status TriangularSolve(asc_sb_context* ctx, const asc_sb_plan* plan, int op, dou
   t.idx = op_csr.idx;
   t.val = op_csr.val;
   t.n = n;
+  t.nnz = op_csr.nnz;
   t.lower = transposed ? triangle == ASC_SB_UPPER : triangle == ASC_SB_LOWER;
   t.unit = diagonal == ASC_SB_UNIT;
   t.conj = op == ASC_SB_OP_CONJUGATE_TRANSPOSE && !RealKind(m->element_kind);
@@ -2014,6 +2015,7 @@ int asc_sb_plan_triangular_analysis(asc_sb_context* ctx, asc_sb_plan* plan, int3
   t.ptr = op_csr.ptr;
   t.idx = op_csr.idx;
   t.n = m.rows;
+  t.nnz = m.nonzeros;
   t.lower = transposed ? triangle == ASC_SB_UPPER : triangle == ASC_SB_LOWER;
   t.control = plan->solve;
   t.status = ctx->status;

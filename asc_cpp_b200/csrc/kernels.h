@@ -227,6 +227,7 @@ typedef struct ascb_trsv {
   const int64_t* idx;
   const void* val;
   int64_t n;
+  int64_t nnz;
   int lower, unit, conj, row_major;
   void* x;
   int64_t ld;

@@ -18,7 +18,14 @@
 // whatever the grid.
 //
 // One right-hand side, short rows: lane i owns the group's i-th row and walks
-// its entries in stored order.  A dependency inside the group is read from
+// its entries in stored order, a batch at a time: the batch's indices, values
+// and positions are fetched before anything is waited for, and its missing
+// values are polled together, so a level costs one hand-over through L2 (about
+// a microsecond) and not a chain of loads per dependency.  What is at hand is
+// used up lane after lane along the group's own chain before the next round of
+// polls.  (One entry at a time, its index and position loaded when its turn
+// came, a level of the 1000^2 Laplacian took 2.05 us, now 1.07 us: 4.09 and
+// 2.14 ms for its 1999 levels, FP64, B200.)  A dependency inside the group is read from
 // shared memory once the owning lane has finished (ballot mask); one outside
 // is read from the published-value array, which holds a signalling-NaN
 // sentinel until the row is solved.  Arithmetic never produces that bit
@@ -69,6 +76,20 @@ constexpr unsigned kFull = 0xffffffffu;
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int64_t kLongRow = 64;
+// Entries of a row that are waited for together, and CTAs per SM the kernel is
+// compiled for.  Level order runs one CTA per SM and has registers to spare.
+// Row order needs rows in flight as much as it needs whole rows in a batch: 3
+// entries (4 CTAs) are best while a row has at most 4 (its diagonal included),
+// 2 entries (5 CTAs) beyond: lower triangle of a 1000^2 5-point Laplacian 3.2
+// against 5.8 ms, of a 100^3 27-point stencil 3.3 against 2.6 ms (FP64, B200;
+// one entry at a time 5.3 and 3.9 ms).
+constexpr int kLevelBatch = 4;
+constexpr int kShortRow = 4;
+constexpr int kShortBatch = 3;
+constexpr int kLongBatch = 2;
+__host__ __device__ constexpr int trsv_ctas(bool levels, int batch) {
+  return levels ? 1 : (batch == kShortBatch ? 4 : 5);
+}
 constexpr uint64_t kWaitNs = 2000000000ull;
 constexpr uint32_t kMaxPolls = 1u << 26;
 
@@ -144,14 +165,18 @@ struct Ar {  // real element arithmetic
   __device__ static T add(T a, T b) { return a + b; }
   __device__ static T load(const T* p) { return __ldg(p); }
   __device__ static T load_l2(const T* p) { return __ldcg(p); }
-  // published value of row c, or false while it is the sentinel
-  __device__ static bool poll(const T* pub, T* out) {
-    using B = Bits<T>;
-    const auto u = ld_relaxed(reinterpret_cast<const typename B::U*>(pub));
-    if (u == B::kSentinel) return false;
-    *out = B::from(u);
+  // a published value as read, and the value, or false while it is the sentinel
+  using Raw = typename Bits<T>::U;
+  __device__ static Raw fetch(const T* pub) {
+    return ld_relaxed(reinterpret_cast<const Raw*>(pub));
+  }
+  __device__ static Raw missing() { return Bits<T>::kSentinel; }
+  __device__ static bool ready(Raw u, T* out) {
+    if (u == Bits<T>::kSentinel) return false;
+    *out = Bits<T>::from(u);
     return true;
   }
+  __device__ static bool poll(const T* pub, T* out) { return ready(fetch(pub), out); }
   __device__ static void publish(T* pub, T v) {
     using B = Bits<T>;
     st_relaxed(reinterpret_cast<typename B::U*>(pub), B::to(v));
@@ -210,16 +235,21 @@ struct Ar<Cx<Rl>> {
   }
   // the two parts are published by separate stores; the value is ready
   // once neither is the sentinel (each part is written once)
-  __device__ static bool poll(const T* pub, T* out) {
+  struct Raw {
+    typename Bits<R>::U re, im;
+  };
+  __device__ static Raw fetch(const T* pub) {
+    const auto* q = reinterpret_cast<const typename Bits<R>::U*>(pub);
+    return {ld_relaxed(q), ld_relaxed(q + 1)};
+  }
+  __device__ static Raw missing() { return {Bits<R>::kSentinel, Bits<R>::kSentinel}; }
+  __device__ static bool ready(Raw u, T* out) {
     using B = Bits<R>;
-    const auto* q = reinterpret_cast<const typename B::U*>(pub);
-    const auto re = ld_relaxed(q);
-    if (re == B::kSentinel) return false;
-    const auto im = ld_relaxed(q + 1);
-    if (im == B::kSentinel) return false;
-    *out = {B::from(re), B::from(im)};
+    if (u.re == B::kSentinel || u.im == B::kSentinel) return false;
+    *out = {B::from(u.re), B::from(u.im)};
     return true;
   }
+  __device__ static bool poll(const T* pub, T* out) { return ready(fetch(pub), out); }
   __device__ static void publish(T* pub, T v) {
     using B = Bits<R>;
     auto* q = reinterpret_cast<typename B::U*>(pub);
@@ -274,11 +304,13 @@ __device__ __forceinline__ int64_t elem(int64_t r, int64_t j, int64_t ld, bool r
   return row_major ? r * ld + j : j * ld + r;
 }
 // Row at solve position s, and solve position of row r.
+template <bool LEVELS>
 __device__ __forceinline__ int64_t row_at(const ascb_trsv& a, int64_t s) {
-  return a.order != nullptr ? __ldg(a.order + s) : (a.lower ? s : a.n - 1 - s);
+  return LEVELS ? __ldg(a.order + s) : (a.lower ? s : a.n - 1 - s);
 }
+template <bool LEVELS>
 __device__ __forceinline__ int64_t position_of(const ascb_trsv& a, int64_t r) {
-  return a.position != nullptr ? __ldg(a.position + r) : (a.lower ? r : a.n - 1 - r);
+  return LEVELS ? __ldg(a.position + r) : (a.lower ? r : a.n - 1 - r);
 }
 __device__ __forceinline__ bool outside(const ascb_trsv& a, int64_t c, int64_t row) {
   return a.lower ? c > row : c < row;
@@ -359,9 +391,10 @@ __device__ void warp_row(const ascb_trsv& a, int64_t row, T alpha, T* pub, Contr
   __syncwarp();
 }
 
-// One right-hand side.
-template <typename T, bool EXACT>
-__global__ void __launch_bounds__(kThreads) trsv_single(ascb_trsv a, T alpha) {
+// One right-hand side; LEVELS: in the level order of an analysis.
+template <typename T, bool EXACT, bool LEVELS, int kBatch>
+__global__ void __launch_bounds__(kThreads, trsv_ctas(LEVELS, kBatch))
+trsv_single(ascb_trsv a, T alpha) {
   using A = Ar<T>;
   __shared__ T solved_value[kWarps][32];
   const int lane = threadIdx.x & 31;
@@ -377,7 +410,7 @@ __global__ void __launch_bounds__(kThreads) trsv_single(ascb_trsv a, T alpha) {
     if (s0 >= a.n) break;
     const int64_t s = s0 + lane;
     const bool valid = s < a.n;
-    const int64_t row = valid ? row_at(a, s) : 0;
+    const int64_t row = valid ? row_at<LEVELS>(a, s) : 0;
     int64_t p = valid ? __ldg(a.ptr + row) : 0;
     const int64_t end = valid ? __ldg(a.ptr + row + 1) : 0;
     if (__any_sync(kFull, end - p > kLongRow)) {
@@ -394,46 +427,102 @@ __global__ void __launch_bounds__(kThreads) trsv_single(ascb_trsv a, T alpha) {
     unsigned solved = 0u;  // lanes whose row is solved
     uint32_t idle = 0;
     uint64_t idle_since = 0;
+    // A batch of entries: index, value and solve position are fetched before
+    // anything is waited for, and all the batch's missing values are polled
+    // together, so that a level costs one hand-over and not a chain of loads
+    // per dependency.
+    int64_t col[kBatch];
+    T v[kBatch], xv[kBatch];
+    int lane_of[kBatch];          // group lane that owns the dependency, or -1
+    unsigned need = 0u, have = 0u;  // dependencies of the batch; those at hand
+    auto open_batch = [&]() {
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) {
+        const bool ok = p + u < end;
+        col[u] = ok ? __ldg(a.idx + p + u) : row;
+        v[u] = ok ? A::load(val + p + u) : A::zero();
+        if (a.conj) v[u] = A::conj(v[u]);
+      }
+      need = have = 0u;
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) {
+        if (p + u < end && col[u] == row) diag = v[u];
+        const bool dep = p + u < end && col[u] != row && !outside(a, col[u], row);
+        lane_of[u] = -1;
+        if (dep) {
+          need |= 1u << u;
+          const int64_t sc = position_of<LEVELS>(a, col[u]);
+          if (sc >= s0 && sc < s0 + 32) lane_of[u] = static_cast<int>(sc - s0);
+        }
+      }
+    };
+    if (!done) open_batch();
     for (;;) {
       bool progressed = false;
       if (!done) {
-        while (p < end) {
-          const int64_t c = __ldg(a.idx + p);
-          T v = A::load(val + p);
-          if (a.conj) v = A::conj(v);
-          if (c == row) {
-            diag = v;
-            ++p;
-            continue;
-          }
-          if (outside(a, c, row)) {
-            ++p;
-            continue;
-          }
-          T xc;
-          const int64_t sc = position_of(a, c);
-          if (sc >= s0 && sc < s0 + 32) {  // earlier lane of this group
-            const int li = static_cast<int>(sc - s0);
-            if (((solved >> li) & 1u) == 0u) break;
-            xc = solved_value[warp][li];
-          } else if (!A::poll(pub + c, &xc)) {
-            break;
-          }
-          value = EXACT ? A::sub(value, A::mul(v, xc)) : A::fms(value, v, xc);
-          ++p;
-          progressed = true;
+        typename A::Raw raw[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          raw[u] = A::missing();
+          if ((((need & ~have) >> u) & 1u) != 0u && lane_of[u] < 0) raw[u] = A::fetch(pub + col[u]);
         }
-        if (p >= end) {
-          if (!a.unit) value = A::div(value, diag);
-          solved_value[warp][lane] = value;
-          x[elem(row, 0, a.ld, row_major)] = value;
-          A::publish(pub + row, value);
-          done = true;
-          progressed = true;
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          if (A::ready(raw[u], &xv[u])) have |= 1u << u;
         }
       }
-      __syncwarp();
-      solved = __ballot_sync(kFull, done);
+      // what is at hand is used up, lane after lane along the group's own
+      // chain, before the next round of polls: a hop between lanes must not
+      // wait for other lanes' polls
+      for (;;) {
+        if (!done) {
+#pragma unroll
+          for (int u = 0; u < kBatch; ++u) {
+            if ((((need & ~have) >> u) & 1u) != 0u && lane_of[u] >= 0 &&
+                ((solved >> lane_of[u]) & 1u) != 0u) {
+              xv[u] = solved_value[warp][lane_of[u]];
+              have |= 1u << u;
+            }
+          }
+          // in stored order: up to the first one that is missing
+#pragma unroll
+          for (int u = 0; u < kBatch; ++u) {
+            const unsigned below = (2u << u) - 1u;
+            if (((need >> u) & 1u) != 0u && ((need & ~have) & below) == 0u) {
+              value = EXACT ? A::sub(value, A::mul(v[u], xv[u])) : A::fms(value, v[u], xv[u]);
+              need &= ~(1u << u);
+              progressed = true;
+            }
+          }
+          if (need == 0u) {
+            p += kBatch;
+            progressed = true;
+            if (p < end) {
+              open_batch();
+            } else {
+              if (!a.unit) value = A::div(value, diag);
+              solved_value[warp][lane] = value;
+              x[elem(row, 0, a.ld, row_major)] = value;
+              A::publish(pub + row, value);
+              done = true;
+            }
+          }
+        }
+        __syncwarp();
+        const unsigned before = solved;
+        solved = __ballot_sync(kFull, done);
+        bool more = solved != before;
+        if (LEVELS) {  // rows of one level wait for others of the group only where levels meet
+          more = false;
+#pragma unroll
+          for (int u = 0; u < kBatch; ++u) {
+            more = more || ((((need & ~have) >> u) & 1u) != 0u && lane_of[u] >= 0 &&
+                            ((solved >> lane_of[u]) & 1u) != 0u);
+          }
+          more = __any_sync(kFull, more);
+        }
+        if (!more) break;
+      }
       if (solved == kFull) break;
       if (__any_sync(kFull, progressed)) {
         idle = 0;
@@ -472,7 +561,8 @@ __global__ void __launch_bounds__(kThreads) trsv_multi(ascb_trsv a, T alpha) {
     if (s0 >= a.n) break;
     const int64_t count = a.n - s0 < 32 ? a.n - s0 : 32;
     for (int64_t i = 0; i < count; ++i) {
-      const int64_t row = row_at(a, s0 + i);
+      const int64_t row =
+          a.order != nullptr ? row_at<true>(a, s0 + i) : row_at<false>(a, s0 + i);
       const int64_t beg = __ldg(a.ptr + row);
       const int64_t end = __ldg(a.ptr + row + 1);
       for (int64_t j0 = 0; j0 < a.k; j0 += 32) {
@@ -695,9 +785,18 @@ int launch_solve(cudaStream_t s, const ascb_trsv& a, T alpha, int sm) {
   const int64_t groups = (a.n + 31) / 32;
   const bool levels = a.order != nullptr;
   if (a.k == 1) {
-    static const int per_sm = Resident(trsv_single<T, EXACT>);
-    const int use = levels ? ASCB_TRSV_LEVEL_CTAS_PER_SM : per_sm;
-    trsv_single<T, EXACT><<<GridFor(groups, kWarps, sm, use), kThreads, 0, s>>>(a, alpha);
+    if (levels) {
+      trsv_single<T, EXACT, true, kLevelBatch>
+          <<<GridFor(groups, kWarps, sm, ASCB_TRSV_LEVEL_CTAS_PER_SM), kThreads, 0, s>>>(a, alpha);
+    } else if (a.nnz <= kShortRow * a.n) {
+      static const int per_sm = Resident(trsv_single<T, EXACT, false, kShortBatch>);
+      trsv_single<T, EXACT, false, kShortBatch>
+          <<<GridFor(groups, kWarps, sm, per_sm), kThreads, 0, s>>>(a, alpha);
+    } else {
+      static const int per_sm = Resident(trsv_single<T, EXACT, false, kLongBatch>);
+      trsv_single<T, EXACT, false, kLongBatch>
+          <<<GridFor(groups, kWarps, sm, per_sm), kThreads, 0, s>>>(a, alpha);
+    }
   } else {
     static const int per_sm = Resident(trsv_multi<T, EXACT>);
     const int use = levels ? ASCB_TRSV_LEVEL_CTAS_PER_SM : per_sm;

@@ -212,4 +212,31 @@ __device__ __forceinline__ int64_t warp_first_row_at(const int64_t* __restrict__
   return lo;
 }
 
+// Two of them side by side, 16 probes a round each: lanes 0..15 get the answer
+// for target0, lanes 16..31 that for target1.
+__device__ __forceinline__ int64_t pair_first_row_at(const int64_t* __restrict__ ptr, int64_t rows,
+                                                     int64_t weight, int64_t target0,
+                                                     int64_t target1, int lane) {
+  const int64_t target = lane < 16 ? target0 : target1;
+  const int probe = lane & 15;
+  int64_t lo = 0;
+  int64_t hi = rows;
+  while (__any_sync(0xffffffffu, lo < hi)) {
+    const int64_t len = hi - lo;
+    const bool last = len <= 16;
+    const int64_t at = last ? lo + probe : lo + len * probe / 16;
+    const bool below = at < hi && weight * at + __ldg(ptr + at) < target;
+    const unsigned votes = __ballot_sync(0xffffffffu, below);
+    const int n = __popc((lane < 16 ? votes : votes >> 16) & 0xffffu);
+    if (last || n == 0) {
+      lo += n;
+      hi = lo;
+    } else {
+      if (n < 16) hi = lo + len * n / 16;
+      lo = lo + len * (n - 1) / 16 + 1;
+    }
+  }
+  return lo;
+}
+
 }  // namespace ascb

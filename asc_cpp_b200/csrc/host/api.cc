@@ -333,7 +333,8 @@ Status RunCsr(asc_sb_context* ctx, const Choice& choice, int form,
     const std::int64_t items = ascb_merge_tile_items();
     const std::int64_t tiles = ascb_row_tile_count(a.rows, a.nnz, items, weight);
     const std::int64_t* tiles_ptr = planned != nullptr ? planned->merge_tiles : nullptr;
-    if (tiles_ptr == nullptr && scratch != nullptr) {
+    if (tiles_ptr == nullptr && scratch != nullptr &&
+        tiles > ascb_seg_one_pass_tiles(ctx->sm_count)) {
       Status s = Launched(ctx, ascb_row_tiles(ctx->stream, &a, items, weight, scratch, tiles),
                           "CUDA could not launch the row-tile partition kernel");
       if (!s.ok()) return s;
@@ -355,7 +356,8 @@ Status RunCsr(asc_sb_context* ctx, const Choice& choice, int form,
   const std::int64_t tiles = ascb_row_tile_count(a.rows, a.nnz, items, weight);
   const std::int64_t* tiles_ptr =
       planned != nullptr ? (seg_aligned ? planned->seg_tiles : planned->warp_tiles) : nullptr;
-  if (tiles_ptr == nullptr && scratch != nullptr) {
+  if (tiles_ptr == nullptr && scratch != nullptr &&
+      !(seg_aligned && tiles <= ascb_seg_one_pass_tiles(ctx->sm_count))) {
     Status s = Launched(ctx,
                         ascb_row_tiles(ctx->stream, &a, items, weight, scratch, tiles),
                         "CUDA could not launch the row-tile partition kernel");

@@ -37,6 +37,7 @@ struct asc_sb_batch {
   std::int64_t count = 0;
   bool unit = true;        // every vector has stride 1
   bool aligned = true;     // every index/value array is 16-byte aligned
+  bool wide = true;        // ... 32-byte aligned
   std::vector<ascb_batch_item> items;  // host copy (per-matrix path)
   ascb_batch_item* items_dev = nullptr;
   std::int64_t* bounds = nullptr;
@@ -79,28 +80,53 @@ class Guard {
   bool ok_ = false;
 };
 
-std::int64_t Tiles(std::int64_t rows, std::int64_t nnz) {
-  return ascb_row_tile_count(rows, nnz, ascb_warp_tile_items(), ascb_warp_tile_row_weight());
+// The row tiles of a batch: the segmented kernel's own (up to 125 rows: banded
+// rows of 30 entries fill 93% of their windows, 80% with at most 32 rows), or
+// the warp kernel's where some array is misaligned.
+std::int64_t TileItems(bool aligned) {
+  return aligned ? ascb_seg_tile_items() : ascb_warp_tile_items();
+}
+std::int64_t TileWeight(bool aligned) {
+  return aligned ? ascb_seg_tile_row_weight() : ascb_warp_tile_row_weight();
+}
+std::int64_t Tiles(std::int64_t rows, std::int64_t nnz, bool aligned) {
+  return ascb_row_tile_count(rows, nnz, TileItems(aligned), TileWeight(aligned));
+}
+bool Aligned(const void* idx, const void* val, std::uintptr_t bytes) {
+  return ((reinterpret_cast<std::uintptr_t>(idx) | reinterpret_cast<std::uintptr_t>(val)) &
+          (bytes - 1)) == 0;
+}
+bool SegAligned(const void* idx, const void* val) {
+  return Aligned(idx, val, static_cast<std::uintptr_t>(ascb_spmv_seg_alignment()));
 }
 
 struct Layout {
   std::size_t items = 0, bounds = 0, queue = 0, total = 0;
   std::int64_t total_tiles = 0, total_bounds = 0;
+  bool aligned = true;
 };
 
 Status LayoutFor(std::int64_t count, const asc_sb_sparse* m, Layout* out) {
   Layout l;
+  // room for either kind of tiles: alignment need not be known when the
+  // workspace is sized
+  std::int64_t tiles[2] = {0, 0};
+  l.aligned = true;
   for (std::int64_t i = 0; i < count; ++i) {
     if (m[i].rows < 0 || m[i].nonzeros < 0) return Fail(ASC_SB_SHAPE, "negative batch extents");
-    const std::int64_t t = m[i].rows > 0 ? Tiles(m[i].rows, m[i].nonzeros) : 0;
-    l.total_tiles += t;
-    l.total_bounds += t + 1;
+    l.aligned = l.aligned && SegAligned(m[i].structure_second, m[i].values);
+    for (int k = 0; k < 2; ++k) {
+      tiles[k] += m[i].rows > 0 ? Tiles(m[i].rows, m[i].nonzeros, k == 1) : 0;
+    }
   }
+  l.total_tiles = tiles[l.aligned ? 1 : 0];
+  l.total_bounds = l.total_tiles + count;
+  const std::int64_t most_bounds = std::max(tiles[0], tiles[1]) + count;
   std::size_t at = 0;
   l.items = at;
   at += RoundUp(static_cast<std::size_t>(count) * sizeof(ascb_batch_item));
   l.bounds = at;
-  at += RoundUp(static_cast<std::size_t>(l.total_bounds) * 8);
+  at += RoundUp(static_cast<std::size_t>(most_bounds) * 8);
   l.queue = at;
   at += RoundUp(8);
   l.total = at;
@@ -124,7 +150,8 @@ int EnqueuePersistent(cudaStream_t stream, const asc_sb_batch& b, int exact, dou
                       double beta, int sm_count) {
   cudaError_t e = cudaMemsetAsync(b.queue, 0, sizeof(unsigned long long), stream);
   if (e != cudaSuccess) return static_cast<int>(e);
-  return ascb_spmv_seg_batch(stream, Dtype(b.element_kind), exact, b.unit ? 1 : 0, b.items_dev,
+  return ascb_spmv_seg_batch(stream, Dtype(b.element_kind), exact, b.unit ? 1 : 0,
+                             b.wide ? 1 : 0, b.items_dev,
                              b.count, b.bounds, b.total_tiles, b.queue, b.chunk, b.ctas_per_sm,
                              alpha, beta, sm_count);
 }
@@ -149,15 +176,14 @@ Status PerMatrix(const ContextView& v, const asc_sb_batch& b, int exact, double 
     a.val = it.val;
     const ascb_vec x{const_cast<void*>(it.x), 0, it.incx};
     const ascb_vec y{it.y, it.rows, it.incy};
-    const std::int64_t tiles = Tiles(it.rows, it.nnz);
+    const std::int64_t tiles = Tiles(it.rows, it.nnz, b.aligned);
     const std::int64_t* tb = b.bounds + it.bound_base;
-    const bool aligned =
-        ((reinterpret_cast<std::uintptr_t>(it.idx) | reinterpret_cast<std::uintptr_t>(it.val)) &
-         static_cast<std::uintptr_t>(ascb_spmv_seg_alignment() - 1)) == 0;
-    const int rc = aligned ? ascb_spmv_seg(v.stream, Dtype(b.element_kind), ASCB_COMPAT, exact, &a,
-                                           alpha, beta, &x, &y, tb, tiles, v.sm_count)
-                           : ascb_spmv_warp(v.stream, Dtype(b.element_kind), ASCB_COMPAT, exact,
-                                            &a, alpha, beta, &x, &y, tb, tiles, v.sm_count);
+    const int rc =
+        SegAligned(it.idx, it.val)
+            ? ascb_spmv_seg_w(v.stream, Dtype(b.element_kind), ASCB_COMPAT, exact, &a, alpha, beta,
+                              &x, &y, tb, tiles, TileWeight(b.aligned), v.sm_count)
+            : ascb_spmv_warp(v.stream, Dtype(b.element_kind), ASCB_COMPAT, exact, &a, alpha, beta,
+                             &x, &y, tb, tiles, v.sm_count);
     Status s = Enqueued(v, rc, "CUDA could not launch a per-matrix SpMV");
     if (!s.ok()) return s;
   }
@@ -240,6 +266,7 @@ int asc_sb_batch_create(asc_sb_context* context, int64_t count, const asc_sb_spa
   auto b = std::make_unique<asc_sb_batch>();
   b->device = v.device;
   b->count = count;
+  b->aligned = l.aligned;
   b->element_kind = count > 0 ? matrices[0].element_kind : ASC_SB_DOUBLE;
   b->items.resize(static_cast<std::size_t>(count));
   std::int64_t tile_base = 0;
@@ -289,12 +316,9 @@ int asc_sb_batch_create(asc_sb_context* context, int64_t count, const asc_sb_spa
     it.incy = outputs[i].stride;
     it.tile_base = tile_base;
     it.bound_base = tile_base + i;
-    tile_base += m.rows > 0 ? Tiles(m.rows, m.nonzeros) : 0;
+    tile_base += m.rows > 0 ? Tiles(m.rows, m.nonzeros, b->aligned) : 0;
     b->unit = b->unit && it.incx == 1 && it.incy == 1;
-    b->aligned = b->aligned &&
-                 ((reinterpret_cast<std::uintptr_t>(it.idx) |
-                   reinterpret_cast<std::uintptr_t>(it.val)) &
-                  static_cast<std::uintptr_t>(ascb_spmv_seg_alignment() - 1)) == 0;
+    b->wide = b->wide && Aligned(it.idx, it.val, 32);
   }
   if (OutputsOverlap(std::move(writes), reads)) {
     return Done(v, Fail(ASC_SB_INVALID_ARGUMENT,
@@ -320,7 +344,8 @@ int asc_sb_batch_create(asc_sb_context* context, int64_t count, const asc_sb_spa
                                     cudaMemcpyHostToDevice, v.stream);
     if (e == cudaSuccess) {
       e = static_cast<cudaError_t>(ascb_batch_tile_bounds(v.stream, b->items_dev, count, b->bounds,
-                                                          b->total_bounds, v.sm_count));
+                                                          b->total_bounds, TileItems(b->aligned),
+                                                    TileWeight(b->aligned), v.sm_count));
       v.launches->fetch_add(1, std::memory_order_relaxed);
     }
     // the host table must outlive the copy: wait for it here (creation is

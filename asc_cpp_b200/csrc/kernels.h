@@ -87,17 +87,16 @@ int64_t ascb_warp_tile_row_weight(void);
 int ascb_spmv_warp(void* stream, int dtype, int form, int exact, const ascb_csr* a,
                    double alpha, double beta, const ascb_vec* x, const ascb_vec* y,
                    const int64_t* tile_row, int64_t ntiles, int sm_count);
-// Register-segmented SpMV over the warp row tiles (exact = 1: bit-exact);
-// requires the column-index and value arrays to start on
+// Register-segmented SpMV (ascb_spmv_seg_w; exact = 1: bit-exact) over row
+// tiles of weight `weight`: ascb_warp_tile_row_weight() (at most 32 rows per
+// tile) or ascb_seg_tile_row_weight() (the segmented kernel's own partition:
+// more rows per tile, so more of each window holds nonzeros when rows are
+// short).  The column-index and value arrays start on
 // ascb_spmv_seg_alignment()-byte boundaries.
 int ascb_spmv_seg_alignment(void);
-int ascb_spmv_seg(void* stream, int dtype, int form, int exact, const ascb_csr* a, double alpha,
-                  double beta, const ascb_vec* x, const ascb_vec* y, const int64_t* tile_row,
-                  int64_t ntiles, int sm_count);
-// The same over row tiles of weight `weight`: ascb_warp_tile_row_weight() (at
-// most 32 rows per tile, as ascb_spmv_seg) or ascb_seg_tile_row_weight() (the
-// segmented kernel's own partition: more rows per tile, so more of each
-// window holds nonzeros when rows are short).
+// Up to this many tiles a NULL tile_row (bounds searched in the kernel) is
+// faster than a partition kernel first.
+int64_t ascb_seg_one_pass_tiles(int sm_count);
 int64_t ascb_seg_tile_row_weight(void);
 // Weighted items per tile of that partition (ascb_row_tiles' `items`): fewer
 // than ascb_warp_tile_items() when the weight is small, so that every row of
@@ -111,7 +110,7 @@ int64_t ascb_merge_tile_items(void);
 int ascb_spmv_seg_w(void* stream, int dtype, int form, int exact, const ascb_csr* a, double alpha,
                     double beta, const ascb_vec* x, const ascb_vec* y, const int64_t* tile_row,
                     int64_t ntiles, int64_t weight, int sm_count);
-// Row split (contracted only): like ascb_spmv_seg with exact = 0, except that
+// Row split (contracted only): like ascb_spmv_seg_w with exact = 0, except that
 // a row running more than split_min (>= 256) positions past its tile's window
 // is finished by a second kernel whose warps take its tail in 256-position
 // chunks; partial sums are combined in chunk order, so results repeat run to
@@ -138,13 +137,16 @@ typedef struct ascb_batch_item {
   int64_t bound_base;   // first entry of its tile bounds (tile_base + index)
 } ascb_batch_item;
 // Tile bounds of every matrix: bounds[bound_base + k] = first row of tile k,
-// k = 0..tiles (the last entry is rows).  `items` is the device table.
+// k = 0..tiles (the last entry is rows), tiles of `items_per_tile` items and row
+// weight `weight`.  `items` is the device table.
 int ascb_batch_tile_bounds(void* stream, const ascb_batch_item* items, int64_t count,
-                           int64_t* bounds, int64_t total_bounds, int sm_count);
+                           int64_t* bounds, int64_t total_bounds, int64_t items_per_tile,
+                           int64_t weight, int sm_count);
 // Persistent work-queue SpMV over all tiles of the batch: warps take `chunk`
 // tiles at a time from *queue (zero before the launch); ctas_per_sm = 0 uses
-// the occupancy limit.  Index and value arrays must be 16-byte aligned.
-int ascb_spmv_seg_batch(void* stream, int dtype, int exact, int unit,
+// the occupancy limit.  The tiles are the segmented kernel's own.  Index and
+// value arrays must be 16-byte aligned (wide = 1: all of them 32-byte aligned).
+int ascb_spmv_seg_batch(void* stream, int dtype, int exact, int unit, int wide,
                         const ascb_batch_item* items, int64_t count, const int64_t* bounds,
                         int64_t total_tiles, unsigned long long* queue, int chunk,
                         int ctas_per_sm, double alpha, double beta, int sm_count);

@@ -88,12 +88,15 @@ struct SplitBlock {
 };
 constexpr unsigned long long kChunkMask = (1ull << 40) - 1;
 
-template <typename T>
+// (Products only where they are staged: shared memory comes out of L1, and the
+// 2 KB a warp cost the contracted kernel 4% on the 4M-row power-law matrix: 504
+// against 486 us, FP64, beta = 0.5, B200.)
+template <typename T, bool EXACT>
 struct SegSmem {
   uint32_t bits[kItems / 32 + 1];  // row-start bitmap of positions 0..256
   int16_t rowid[32 * 8 + 1];       // k-th nonempty row of the tile -> its offset (RPL <= 8)
   int64_t bnd[kChunk + 1];         // first row of tiles c0 .. c0 + kChunk
-  alignas(16) T prod[kItems];      // exact form: the window's / a long row's products
+  alignas(16) T prod[EXACT ? kItems : 1];  // the window's / a long row's products
 };
 
 // Arithmetic of the two modes.  EXACT rounds every product and sum separately
@@ -293,7 +296,7 @@ __device__ __forceinline__ float chain_sum(float acc, const float* prod, int q, 
 // the instruction count per tile follows the longest row, not the number of
 // lane boundaries the rows cross.
 template <typename T, bool STANDARD, bool UNIT, bool V32, int RPL>
-__device__ __forceinline__ void exact_tile(SegSmem<T>& w, int lane,
+__device__ __forceinline__ void exact_tile(SegSmem<T, true>& w, int lane,
                                            const int64_t* __restrict__ ptr,
                                            const int64_t* __restrict__ idx,
                                            const T* __restrict__ val, const T* __restrict__ x,
@@ -369,7 +372,7 @@ __device__ __forceinline__ void exact_tile(SegSmem<T>& w, int lane,
 // single-matrix and the batched kernels.
 template <typename T, bool EXACT, bool STANDARD, bool UNIT, bool SPLIT = false, bool V32 = false,
           int RPL = 1>
-__device__ __forceinline__ void seg_tile(SegSmem<T>& w, int lane, const int64_t* __restrict__ ptr,
+__device__ __forceinline__ void seg_tile(SegSmem<T, EXACT>& w, int lane, const int64_t* __restrict__ ptr,
                                          const int64_t* __restrict__ idx,
                                          const T* __restrict__ val, const T* __restrict__ x,
                                          int64_t incx, T* __restrict__ y, int64_t incy, T alpha,
@@ -607,9 +610,9 @@ seg_kernel(const int64_t* __restrict__ ptr, const int64_t* __restrict__ idx,
            const T* __restrict__ val, const T* __restrict__ x, int64_t incx, T* __restrict__ y,
            int64_t incy, T alpha, T beta, const int64_t* __restrict__ tile_row, int64_t ntiles,
            int64_t rows, int64_t nnz, SplitBlock split) {
-  __shared__ SegSmem<T> smem_all[kWarpsPerCta];
+  __shared__ SegSmem<T, EXACT> smem_all[kWarpsPerCta];
   const int lane = threadIdx.x & 31;
-  SegSmem<T>& w = smem_all[threadIdx.x >> 5];
+  SegSmem<T, EXACT>& w = smem_all[threadIdx.x >> 5];
 
   const int64_t warp_id = static_cast<int64_t>(blockIdx.x) * kWarpsPerCta + (threadIdx.x >> 5);
   const int64_t warp_count = static_cast<int64_t>(gridDim.x) * kWarpsPerCta;
@@ -641,7 +644,15 @@ seg_kernel(const int64_t* __restrict__ ptr, const int64_t* __restrict__ idx,
   // prefetch of the next tile's row bounds (one round trip ahead)
   int64_t r0_n;
   int nr_n;
-  tile_bounds(tb, r0_n, nr_n);
+  if (tile_row == nullptr && per_warp == 1) {  // its only tile: both bounds at once
+    const int64_t b = pair_first_row_at(ptr, rows, kRowWeight / RPL, tb * tile_items<RPL>(),
+                                        te * tile_items<RPL>(), lane);
+    r0_n = __shfl_sync(0xffffffffu, b, 0);
+    const int64_t end = __shfl_sync(0xffffffffu, b, 16);
+    nr_n = static_cast<int>((te < ntiles ? end : rows) - r0_n);
+  } else {
+    tile_bounds(tb, r0_n, nr_n);
+  }
   int64_t rb_n = lane < nr_n ? __ldg(ptr + r0_n + lane) : 0;
   int64_t re_n = lane < nr_n ? __ldg(ptr + r0_n + lane + 1) : 0;
 
@@ -734,23 +745,27 @@ split_chunk_kernel(const int64_t* __restrict__ idx, const T* __restrict__ val,
 // ---- batched: many independent matrices in one persistent launch ---------
 
 // Last matrix whose first global tile is <= t (matrices without tiles share
-// their successor's first tile and are skipped this way).
+// their successor's first tile and are skipped this way), by the whole warp:
+// 32 probes a round, two rounds for a thousand matrices.
 __device__ __forceinline__ int64_t batch_matrix_of(const ascb_batch_item* __restrict__ items,
-                                                   int64_t count, int64_t t) {
-  int64_t lo = 0, hi = count - 1;
-  while (lo < hi) {
-    const int64_t mid = (lo + hi + 1) >> 1;
-    if (__ldg(&items[mid].tile_base) <= t) {
-      lo = mid;
-    } else {
-      hi = mid - 1;
-    }
+                                                   int64_t count, int64_t t, int lane) {
+  int64_t lo = 0, hi = count;  // the answer lies in [lo, hi)
+  while (hi - lo > 1) {
+    const int64_t len = hi - lo;
+    const bool last = len <= 32;
+    const int64_t at = last ? lo + lane : lo + len * lane / 32;
+    const bool here = at < hi && __ldg(&items[at].tile_base) <= t;
+    const int n = __popc(__ballot_sync(0xffffffffu, here));  // at least 1: items[lo] qualifies
+    if (last) return lo + n - 1;
+    if (n < 32) hi = lo + len * n / 32;
+    lo = lo + len * (n - 1) / 32;
   }
   return lo;
 }
 
 __global__ void batch_bounds_kernel(const ascb_batch_item* __restrict__ items, int64_t count,
-                                    int64_t* __restrict__ bounds, int64_t total_bounds) {
+                                    int64_t* __restrict__ bounds, int64_t total_bounds,
+                                    int64_t tile, int64_t weight) {
   const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < total_bounds;
        e += step) {
@@ -768,39 +783,52 @@ __global__ void batch_bounds_kernel(const ascb_batch_item* __restrict__ items, i
     const int64_t tiles = next - __ldg(&it.bound_base) - 1;
     const int64_t k = e - __ldg(&it.bound_base);
     bounds[e] = k >= tiles ? __ldg(&it.rows)
-                           : first_row_at(it.ptr, __ldg(&it.rows), kRowWeight, k * kItems);
+                           : first_row_at(it.ptr, __ldg(&it.rows), weight, k * tile);
   }
 }
 
-template <typename T, bool EXACT, bool UNIT>
+// (512 banded matrices of up to 16,384 rows, half bandwidth up to 31, FP64, B200:
+// 612 us on tiles of at most 32 rows with 16-byte loads and nothing asked for
+// early, 572 us; bit-exact 707 and 630; half bandwidth up to 5 218 and 168.  The
+// DRAM floor of the first is 358 us: latency, 28 warps an SM at 72 registers.)
+// Warps take `chunk` consecutive tiles at a time.  What a tile needs is asked for
+// a step early: the next ticket while the current tiles run, the next tile's
+// bounds and row offsets (same matrix) while the current tile runs.
+template <typename T, bool EXACT, bool UNIT, bool V32>
 __global__ void __launch_bounds__(kThreads, EXACT ? kMinCtasExact : kMinCtasFast)
 seg_batch_kernel(const ascb_batch_item* __restrict__ items, int64_t count,
                  const int64_t* __restrict__ bounds, int64_t total_tiles,
                  unsigned long long* __restrict__ queue, int chunk, T alpha, T beta) {
-  __shared__ SegSmem<T> smem_all[kWarpsPerCta];
+  __shared__ SegSmem<T, EXACT> smem_all[kWarpsPerCta];
   const int lane = threadIdx.x & 31;
-  SegSmem<T>& w = smem_all[threadIdx.x >> 5];
-  int64_t tile_lo = 0, tile_hi = 0, bound_base = 0;
+  SegSmem<T, EXACT>& w = smem_all[threadIdx.x >> 5];
+  int64_t tile_lo = 0, tile_hi = 0, bound_base = 0, rows = 0;
   const int64_t* ptr = nullptr;
   const int64_t* idx = nullptr;
   const T* val = nullptr;
   const T* x = nullptr;
   T* y = nullptr;
   int64_t incx = 1, incy = 1;
+  unsigned long long ticket = 0;
+  const int64_t share = static_cast<int64_t>(gridDim.x) * kWarpsPerCta * chunk;  // one of each
+  if (lane == 0) ticket = atomicAdd(queue, static_cast<unsigned long long>(chunk));
   for (;;) {
-    unsigned long long t0 = 0;
-    if (lane == 0) t0 = atomicAdd(queue, static_cast<unsigned long long>(chunk));
-    t0 = __shfl_sync(0xffffffffu, t0, 0);
-    if (t0 >= static_cast<unsigned long long>(total_tiles)) break;
-    const int64_t t1 = static_cast<int64_t>(t0) + chunk < total_tiles
-                           ? static_cast<int64_t>(t0) + chunk : total_tiles;
-    for (int64_t t = static_cast<int64_t>(t0); t < t1; ++t) {
+    const int64_t t0 = static_cast<int64_t>(__shfl_sync(0xffffffffu, ticket, 0));
+    if (t0 >= total_tiles) break;
+    // (not near the end: a warp must not hold tiles that others could take)
+    const bool early = t0 + 2 * share < total_tiles;
+    if (early && lane == 0) ticket = atomicAdd(queue, static_cast<unsigned long long>(chunk));
+    const int64_t t1 = t0 + chunk < total_tiles ? t0 + chunk : total_tiles;
+    int64_t r0 = 0, r1 = 0, rb = 0, re = 0;
+    bool ready = false;  // they are those of tile t
+    for (int64_t t = t0; t < t1; ++t) {
       if (t < tile_lo || t >= tile_hi) {
-        const int64_t m = batch_matrix_of(items, count, t);
+        const int64_t m = batch_matrix_of(items, count, t, lane);
         const ascb_batch_item& it = items[m];
         tile_lo = __ldg(&it.tile_base);
         tile_hi = m + 1 < count ? __ldg(&items[m + 1].tile_base) : total_tiles;
         bound_base = __ldg(&it.bound_base);
+        rows = __ldg(&it.rows);
         ptr = it.ptr;
         idx = it.idx;
         val = static_cast<const T*>(it.val);
@@ -808,16 +836,30 @@ seg_batch_kernel(const ascb_batch_item* __restrict__ items, int64_t count,
         y = static_cast<T*>(it.y);
         incx = __ldg(&it.incx);
         incy = __ldg(&it.incy);
+        ready = false;
       }
-      const int64_t k = bound_base + (t - tile_lo);
-      const int64_t r0 = __ldg(bounds + k);
-      const int nr = static_cast<int>(__ldg(bounds + k + 1) - r0);
+      const int64_t* b = bounds + bound_base + (t - tile_lo);
+      if (!ready) {
+        r0 = __ldg(b);
+        r1 = __ldg(b + 1);
+        rb = __ldg(ptr + (r0 + lane < rows ? r0 + lane : rows));
+        re = __ldg(ptr + (r0 + lane < rows ? r0 + lane + 1 : rows));
+      }
+      const int64_t cur = r0, cur_b = rb, cur_e = re;
+      const int nr = static_cast<int>(r1 - r0);
+      ready = t + 1 < t1 && t + 1 < tile_hi;
+      if (ready) {
+        r0 = r1;
+        r1 = __ldg(b + 2);
+        rb = __ldg(ptr + (r0 + lane < rows ? r0 + lane : rows));
+        re = __ldg(ptr + (r0 + lane < rows ? r0 + lane + 1 : rows));
+      }
       if (nr == 0) continue;
-      const int64_t rb = lane < nr ? __ldg(ptr + r0 + lane) : 0;
-      const int64_t re = lane < nr ? __ldg(ptr + r0 + lane + 1) : 0;
-      seg_tile<T, EXACT, false, UNIT>(w, lane, ptr, idx, val, x, incx, y, incy, alpha, beta, r0, nr,
-                                      rb, re);
+      seg_tile<T, EXACT, false, UNIT, false, V32, kMaxRowsPerLane>(
+          w, lane, ptr, idx, val, x, incx, y, incy, alpha, beta, cur, nr,
+          lane < nr ? cur_b : 0, lane < nr ? cur_e : 0);
     }
+    if (!early && lane == 0) ticket = atomicAdd(queue, static_cast<unsigned long long>(chunk));
   }
 }
 
@@ -849,8 +891,7 @@ template <typename T, bool EXACT, bool STANDARD, bool UNIT, bool V32, int RPL>
 int launch_v(cudaStream_t stream, const ascb_csr* a, T alpha, T beta, const ascb_vec* x,
              const ascb_vec* y, const int64_t* tile_row, int64_t ntiles, int sm_count) {
   auto kernel = seg_kernel<T, EXACT, STANDARD, UNIT, false, V32, RPL>;
-  const int64_t warps_needed = (ntiles + 3) / 4;
-  const int64_t ctas_needed = (warps_needed + kWarpsPerCta - 1) / kWarpsPerCta;
+  const int64_t ctas_needed = (ntiles + kWarpsPerCta - 1) / kWarpsPerCta;  // a tile a warp
   const int64_t resident_ctas = static_cast<int64_t>(sm_count > 0 ? sm_count : 148) *
                                 resident<T, EXACT, STANDARD, UNIT, (V32 ? 4 : 0) + 16 * RPL>(kernel);
   const unsigned blocks = static_cast<unsigned>(
@@ -877,8 +918,7 @@ int launch_split_v(cudaStream_t stream, const ascb_csr* a, T alpha, T beta, cons
                    const ascb_vec* y, const int64_t* tile_row, int64_t ntiles, int sm_count,
                    const SplitBlock& split) {
   auto kernel = seg_kernel<T, false, STANDARD, UNIT, true, V32, RPL>;
-  const int64_t warps_needed = (ntiles + 3) / 4;
-  const int64_t ctas_needed = (warps_needed + kWarpsPerCta - 1) / kWarpsPerCta;
+  const int64_t ctas_needed = (ntiles + kWarpsPerCta - 1) / kWarpsPerCta;  // a tile a warp
   const int per_sm = resident<T, false, STANDARD, UNIT, (V32 ? 5 : 2) + 16 * RPL>(kernel);
   const int64_t resident_ctas = static_cast<int64_t>(sm_count > 0 ? sm_count : 148) * per_sm;
   const unsigned blocks = static_cast<unsigned>(
@@ -953,14 +993,6 @@ int seg_rows(void* stream, int dtype, int form, int exact, const ascb_csr* a, do
 }  // namespace
 }  // namespace ascb
 
-extern "C" int ascb_spmv_seg(void* stream, int dtype, int form, int exact, const ascb_csr* a,
-                             double alpha, double beta, const ascb_vec* x, const ascb_vec* y,
-                             const int64_t* tile_row, int64_t ntiles, int sm_count) {
-  if (ntiles <= 0) return 0;
-  return ascb::seg_rows<1>(stream, dtype, form, exact, a, alpha, beta, x, y, tile_row, ntiles,
-                           sm_count);
-}
-
 extern "C" int64_t ascb_seg_tile_row_weight(void) { return ascb::kSegWeight; }
 extern "C" int64_t ascb_seg_tile_items(void) {
   return ascb::tile_items<ascb::kMaxRowsPerLane>();
@@ -991,6 +1023,16 @@ extern "C" int ascb_spmv_seg_w(void* stream, int dtype, int form, int exact, con
 }
 
 extern "C" int ascb_spmv_seg_alignment(void) { return 16; }
+
+// With this many tiles or fewer every warp has one, all at once, and finds its
+// bounds itself (two 16-way searches side by side) in less time than a
+// partition kernel ahead of it takes: y = A x + y / 2 on the 316^2 Laplacian,
+// FP64, bit-exact, B200: 20.6 us with a partition and four tiles to a warp,
+// 8.3 us (DRAM floor 1.7).
+extern "C" int64_t ascb_seg_one_pass_tiles(int sm_count) {
+  return static_cast<int64_t>(sm_count > 0 ? sm_count : 148) * ascb::kMinCtasExact *
+         ascb::kWarpsPerCta;
+}
 
 namespace ascb {
 namespace {
@@ -1078,16 +1120,19 @@ extern "C" int ascb_spmv_split(void* stream, int dtype, int form, const ascb_csr
 namespace ascb {
 namespace {
 
-template <typename T, bool EXACT, bool UNIT>
+template <typename T, bool EXACT, bool UNIT, bool V32>
 int launch_batch(cudaStream_t s, const ascb_batch_item* items, int64_t count,
                  const int64_t* bounds, int64_t total_tiles, unsigned long long* queue, int chunk,
                  int ctas_per_sm, T alpha, T beta, int sm) {
-  auto kernel = seg_batch_kernel<T, EXACT, UNIT>;
+  auto kernel = seg_batch_kernel<T, EXACT, UNIT, V32>;
   int per_sm = ctas_per_sm;
-  if (per_sm <= 0) per_sm = resident<T, EXACT, false, UNIT, 1>(kernel);
+  if (per_sm <= 0) per_sm = resident<T, EXACT, false, UNIT, V32 ? 7 : 1>(kernel);
+  const int64_t cap = static_cast<int64_t>(sm > 0 ? sm : 148) * per_sm;
+  // no more tiles at a time than leave every resident warp some
+  const int64_t share = (total_tiles + cap * kWarpsPerCta - 1) / (cap * kWarpsPerCta);
+  if (chunk > share) chunk = static_cast<int>(share);
   const int64_t warps_needed = (total_tiles + chunk - 1) / chunk;
   const int64_t ctas_needed = (warps_needed + kWarpsPerCta - 1) / kWarpsPerCta;
-  const int64_t cap = static_cast<int64_t>(sm > 0 ? sm : 148) * per_sm;
   const unsigned blocks =
       static_cast<unsigned>(ctas_needed < 1 ? 1 : (ctas_needed < cap ? ctas_needed : cap));
   kernel<<<blocks, kThreads, 0, s>>>(items, count, bounds, total_tiles, queue, chunk, alpha, beta);
@@ -1095,38 +1140,44 @@ int launch_batch(cudaStream_t s, const ascb_batch_item* items, int64_t count,
 }
 
 template <typename T>
-int batch_typed(cudaStream_t s, int exact, int unit, const ascb_batch_item* items, int64_t count,
-                const int64_t* bounds, int64_t total_tiles, unsigned long long* queue, int chunk,
-                int ctas, double alpha, double beta, int sm) {
+int batch_typed(cudaStream_t s, int exact, int unit, int wide, const ascb_batch_item* items,
+                int64_t count, const int64_t* bounds, int64_t total_tiles,
+                unsigned long long* queue, int chunk, int ctas, double alpha, double beta, int sm) {
   const T a = static_cast<T>(alpha), b = static_cast<T>(beta);
+#define ASCB_BATCH(E, U, V)                                                                     \
+  return launch_batch<T, E, U, V>(s, items, count, bounds, total_tiles, queue, chunk, ctas, a, \
+                                  b, sm)
   if (exact) {
-    return unit ? launch_batch<T, true, true>(s, items, count, bounds, total_tiles, queue, chunk,
-                                              ctas, a, b, sm)
-                : launch_batch<T, true, false>(s, items, count, bounds, total_tiles, queue, chunk,
-                                               ctas, a, b, sm);
+    if (unit && wide) ASCB_BATCH(true, true, true);
+    if (unit) ASCB_BATCH(true, true, false);
+    if (wide) ASCB_BATCH(true, false, true);
+    ASCB_BATCH(true, false, false);
   }
-  return unit ? launch_batch<T, false, true>(s, items, count, bounds, total_tiles, queue, chunk,
-                                             ctas, a, b, sm)
-              : launch_batch<T, false, false>(s, items, count, bounds, total_tiles, queue, chunk,
-                                              ctas, a, b, sm);
+  if (unit && wide) ASCB_BATCH(false, true, true);
+  if (unit) ASCB_BATCH(false, true, false);
+  if (wide) ASCB_BATCH(false, false, true);
+  ASCB_BATCH(false, false, false);
+#undef ASCB_BATCH
 }
 
 }  // namespace
 }  // namespace ascb
 
 extern "C" int ascb_batch_tile_bounds(void* stream, const ascb_batch_item* items, int64_t count,
-                                      int64_t* bounds, int64_t total_bounds, int sm_count) {
+                                      int64_t* bounds, int64_t total_bounds, int64_t items_per_tile,
+                                      int64_t weight, int sm_count) {
   if (count <= 0 || total_bounds <= 0) return 0;
   int64_t blocks = (total_bounds + 255) / 256;
   const int64_t cap = static_cast<int64_t>(sm_count > 0 ? sm_count : 148) * 8;
   if (blocks > cap) blocks = cap;
   ascb::batch_bounds_kernel<<<static_cast<unsigned>(blocks), 256, 0,
                               static_cast<cudaStream_t>(stream)>>>(items, count, bounds,
-                                                                  total_bounds);
+                                                                  total_bounds, items_per_tile,
+                                                                  weight);
   return static_cast<int>(cudaGetLastError());
 }
 
-extern "C" int ascb_spmv_seg_batch(void* stream, int dtype, int exact, int unit,
+extern "C" int ascb_spmv_seg_batch(void* stream, int dtype, int exact, int unit, int wide,
                                    const ascb_batch_item* items, int64_t count,
                                    const int64_t* bounds, int64_t total_tiles,
                                    unsigned long long* queue, int chunk, int ctas_per_sm,
@@ -1135,9 +1186,9 @@ extern "C" int ascb_spmv_seg_batch(void* stream, int dtype, int exact, int unit,
   if (chunk < 1) chunk = 1;
   auto s = static_cast<cudaStream_t>(stream);
   if (dtype == ASCB_F64) {
-    return ascb::batch_typed<double>(s, exact, unit, items, count, bounds, total_tiles, queue,
+    return ascb::batch_typed<double>(s, exact, unit, wide, items, count, bounds, total_tiles, queue,
                                      chunk, ctas_per_sm, alpha, beta, sm_count);
   }
-  return ascb::batch_typed<float>(s, exact, unit, items, count, bounds, total_tiles, queue, chunk,
-                                  ctas_per_sm, alpha, beta, sm_count);
+  return ascb::batch_typed<float>(s, exact, unit, wide, items, count, bounds, total_tiles, queue,
+                                  chunk, ctas_per_sm, alpha, beta, sm_count);
 }

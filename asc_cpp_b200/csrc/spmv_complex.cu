@@ -3,14 +3,21 @@
 // Every stored entry does out += (alpha * v') * in, v' = conj(v) for the
 // conjugate transpose (include/asc/sparse/blas.h:1653-1665 and 1739-1748,
 // MaybeConjugate).  Arrays hold (re, im) pairs, the layout of std::complex<R>,
-// aligned to R only, so components are loaded one by one.  A complex product
+// aligned to R only; where the arrays happen to start on whole elements a pair is
+// one load.  A complex product
 // (a, b)(c, d) is (ac - bd, ad + bc); in EXACT mode every product, difference
 // and sum is rounded separately (the value std::complex<R> gives under GCC
 // without -march for every product that is not NaN + NaN i).
 //   * row products: the CSR arrays handed in are the rows of op(A) (for a
-//     transposed product, the transposed structure of a plan).  One warp per
-//     row, 32 products at a time; EXACT adds them to y one by one in stored
-//     order, FAST sums the row with a warp tree and adds it to y once.
+//     transposed product, the transposed structure of a plan).  A warp takes up
+//     to 32 consecutive rows, whose entries lie one behind the other: all lanes
+//     form 128 products at a time in shared memory while the next 128 entries
+//     are on their way, and each row's lane adds its own in stored order (EXACT
+//     to y, FAST to a sum that y gets once, rounds inside one row by a warp
+//     tree).  With a warp per row and the products
+//     handed to one sum by shuffles, rows of 27 entries left lanes idle and
+//     cost 4 x 27 dependent steps: 27-point stencil on 63^3, Z, bit-exact, B200:
+//     167 us, now 47 (DRAM floor 26).
 //   * scatter: FAST transposed products without a plan, one warp per stored
 //     row, atomic adds of both components.
 //   * SpMM: one thread per (row, right-hand side) in stored order, or the
@@ -55,47 +62,111 @@ __device__ __forceinline__ Cx<R> stored(const Cx<R>* val, int64_t q) {
   return v;
 }
 
-template <typename R>
-__device__ __forceinline__ Cx<R> shfl(Cx<R> v, int src) {
-  return {__shfl_sync(0xffffffffu, v.re, src), __shfl_sync(0xffffffffu, v.im, src)};
+// A whole element at a time (PAIR: on whole-element boundaries).
+template <bool PAIR>
+__device__ __forceinline__ Cx<double> fetch(const Cx<double>* p) {
+  if (!PAIR) return load(p);
+  const double2 v = __ldg(reinterpret_cast<const double2*>(p));
+  return {v.x, v.y};
+}
+template <bool PAIR>
+__device__ __forceinline__ Cx<float> fetch(const Cx<float>* p) {
+  if (!PAIR) return load(p);
+  const float2 v = __ldg(reinterpret_cast<const float2*>(p));
+  return {v.x, v.y};
 }
 
-template <typename R, bool EXACT, bool CONJ, bool UNIT>
+constexpr int kPer = 4;             // products per lane and round
+constexpr int kRound = 32 * kPer;   // 128
+
+template <typename R, bool EXACT, bool CONJ, bool UNIT, bool PAIR>
 __global__ void __launch_bounds__(kThreads)
 complex_rows(const int64_t* __restrict__ ptr, const int64_t* __restrict__ idx,
              const Cx<R>* __restrict__ val, const Cx<R>* __restrict__ x, int64_t incx,
-             Cx<R>* __restrict__ y, int64_t incy, Cx<R> alpha, int64_t rows) {
+             Cx<R>* __restrict__ y, int64_t incy, Cx<R> alpha, int64_t rows, int per_warp) {
+  __shared__ Cx<R> staged[kThreads / 32][kRound];
+  Cx<R>* prod = staged[threadIdx.x / 32];
   const int lane = threadIdx.x & 31;
   const int64_t warps = static_cast<int64_t>(gridDim.x) * (kThreads / 32);
-  for (int64_t r = (static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 5; r < rows;
-       r += warps) {
-    const int64_t b = __ldg(ptr + r);
-    const int64_t e = __ldg(ptr + r + 1);
-    if (b == e) continue;  // no entry: y keeps its bits
-    Cx<R>* yp = &at<UNIT>(y, r, incy);
-    Cx<R> s = EXACT ? *yp : Cx<R>{R(0), R(0)};
-    for (int64_t q0 = b; q0 < e; q0 += 32) {
-      const int64_t q = q0 + lane;
-      Cx<R> p{R(0), R(0)};
-      if (q < e) {
-        const Cx<R> xv = load(&at<UNIT>(x, __ldg(idx + q), incx));
-        p = cmul<EXACT>(cmul<EXACT>(alpha, stored<CONJ>(val, q)), xv);
+  for (int64_t r0 = (static_cast<int64_t>(blockIdx.x) * (kThreads / 32) + threadIdx.x / 32) *
+                    per_warp;
+       r0 < rows; r0 += warps * per_warp) {
+    const int64_t last = r0 + per_warp < rows ? r0 + per_warp : rows;
+    const int64_t r = r0 + lane;
+    const bool mine = r < last;
+    const int64_t end = __ldg(ptr + last);
+    const int64_t b = mine ? __ldg(ptr + r) : end;
+    const int64_t e = mine ? __ldg(ptr + r + 1) : end;
+    const int64_t begin = __shfl_sync(0xffffffffu, b, 0);
+    Cx<R> s{R(0), R(0)};
+    if (EXACT && b < e) s = at<UNIT>(y, r, incy);
+    int64_t col[kPer];
+    Cx<R> v[kPer];
+    auto entries = [&](int64_t w) {
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        const int64_t q = w + u * 32 + lane;
+        if (q < end) {
+          col[u] = __ldg(idx + q);
+          v[u] = fetch<PAIR>(val + q);
+          if (CONJ) v[u].im = -v[u].im;
+        }
       }
-      if (EXACT) {
-        const int n = static_cast<int>(e - q0 < 32 ? e - q0 : 32);
-        for (int k = 0; k < n; ++k) s = cadd<true>(s, shfl(p, k));
-      } else {
-        s = cadd<false>(s, p);
-      }
-    }
-    if (!EXACT) {
+    };
+    Cx<R> wide{R(0), R(0)};  // FAST: this lane's share of a long row, and that row's lane
+    int owner = -1;
+    auto join = [&]() {
+      if (owner < 0) return;
 #pragma unroll
       for (int m = 16; m > 0; m >>= 1) {
-        s.re += __shfl_xor_sync(0xffffffffu, s.re, m);
-        s.im += __shfl_xor_sync(0xffffffffu, s.im, m);
+        wide.re += __shfl_xor_sync(0xffffffffu, wide.re, m);
+        wide.im += __shfl_xor_sync(0xffffffffu, wide.im, m);
       }
+      if (lane == owner) s = cadd<false>(s, wide);
+      wide = {R(0), R(0)};
+      owner = -1;
+    };
+    entries(begin);
+    for (int64_t w = begin; w < end; w += kRound) {
+      Cx<R> xv[kPer];
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        if (w + u * 32 + lane < end) xv[u] = fetch<PAIR>(&at<UNIT>(x, col[u], incx));
+      }
+      if constexpr (!EXACT) {
+        // a round wholly inside one row: every lane keeps its own sum
+        const unsigned whole = __ballot_sync(0xffffffffu, b <= w && e - w >= kRound);
+        if (whole != 0u) {
+          if (owner >= 0 && owner != __ffs(whole) - 1) join();
+#pragma unroll
+          for (int u = 0; u < kPer; ++u) {
+            wide = cadd<false>(wide, cmul<false>(cmul<false>(alpha, v[u]), xv[u]));
+          }
+          owner = __ffs(whole) - 1;
+          if (w + kRound < end) entries(w + kRound);
+          continue;
+        }
+        join();
+      }
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        if (w + u * 32 + lane < end) {
+          prod[u * 32 + lane] = cmul<EXACT>(cmul<EXACT>(alpha, v[u]), xv[u]);
+        }
+      }
+      if (w + kRound < end) entries(w + kRound);
+      __syncwarp();
+      const int from = static_cast<int>((b > w ? b : w) - w);
+      const int64_t to = e - w < kRound ? e - w : kRound;
+#pragma unroll 4
+      for (int q = from; q < to; ++q) s = cadd<EXACT>(s, prod[q]);
+      __syncwarp();  // the products are replaced
     }
-    if (lane == 0) *yp = EXACT ? s : cadd<false>(*yp, s);
+    if constexpr (!EXACT) join();
+    if (b < e) {  // (without entries y keeps its bits)
+      Cx<R>* yp = &at<UNIT>(y, r, incy);
+      *yp = EXACT ? s : cadd<false>(*yp, s);
+    }
   }
 }
 
@@ -189,17 +260,27 @@ int spmv_typed(cudaStream_t s, int mode, const ascb_csr* a, Cx<R> alpha, const a
   const auto* val = static_cast<const Cx<R>*>(a->val);
   const auto* xd = static_cast<const Cx<R>*>(x->data);
   auto* yd = static_cast<Cx<R>*>(y->data);
-  const unsigned blocks = Blocks(a->rows * 32, sm);
   if (mode == 2) {
-    complex_scatter<R, CONJ, UNIT><<<blocks, kThreads, 0, s>>>(ptr, idx, val, xd, x->stride, yd,
-                                                               y->stride, alpha, a->rows);
-  } else if (mode == 1) {
-    complex_rows<R, true, CONJ, UNIT><<<blocks, kThreads, 0, s>>>(ptr, idx, val, xd, x->stride,
-                                                                  yd, y->stride, alpha, a->rows);
-  } else {
-    complex_rows<R, false, CONJ, UNIT><<<blocks, kThreads, 0, s>>>(ptr, idx, val, xd, x->stride,
-                                                                   yd, y->stride, alpha, a->rows);
+    complex_scatter<R, CONJ, UNIT><<<Blocks(a->rows * 32, sm), kThreads, 0, s>>>(
+        ptr, idx, val, xd, x->stride, yd, y->stride, alpha, a->rows);
+    return static_cast<int>(cudaGetLastError());
   }
+  const bool pair = ((reinterpret_cast<uintptr_t>(val) | reinterpret_cast<uintptr_t>(xd)) &
+                     (sizeof(Cx<R>) - 1)) == 0;
+  // as many rows a warp as still leave every SM 16 warps, but no more entries
+  // than four rounds' worth on average, nor a little more than one
+  const int64_t mean = a->nnz / a->rows + 1;
+  int64_t per_warp = a->rows / (static_cast<int64_t>(sm > 0 ? sm : 148) * 16);
+  if (per_warp * mean > 4 * kRound) per_warp = 4 * kRound / mean;
+  if (per_warp * mean > kRound && per_warp * mean < 2 * kRound) per_warp = kRound / mean;
+  per_warp = per_warp < 1 ? 1 : (per_warp > 32 ? 32 : per_warp);
+  const unsigned blocks = Blocks((a->rows + per_warp - 1) / per_warp * 32, sm);
+  auto kernel = mode == 1 ? (pair ? complex_rows<R, true, CONJ, UNIT, true>
+                                  : complex_rows<R, true, CONJ, UNIT, false>)
+                          : (pair ? complex_rows<R, false, CONJ, UNIT, true>
+                                  : complex_rows<R, false, CONJ, UNIT, false>);
+  kernel<<<blocks, kThreads, 0, s>>>(ptr, idx, val, xd, x->stride, yd, y->stride, alpha, a->rows,
+                                     static_cast<int>(per_warp));
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -56,12 +56,23 @@ __host__ __device__ constexpr int64_t tile_items() {
 constexpr int kPer = 8;            // contiguous positions per lane
 constexpr int kChunk = 32;         // tile bounds cached per warp
 constexpr int kMaxDevices = 64;
-// CTAs per SM the segmented kernels are compiled for (register cap): on the
-// 4M-row power-law matrix (B200) the contracted tile runs best at 7 (72
-// registers: 2621 / 2667 GB/s plain / row split, against 2567 / 2524 at 6),
-// the bit-exact tile at 6 (2250 against 2168 GB/s at 7, and 1895 at 5).
-constexpr int kMinCtasFast = 7;
-constexpr int kMinCtasExact = 6;
+// CTAs per SM the segmented kernels are compiled for (register cap).  Warps in
+// flight hide the gathers; spills and shared memory out of L1 cost.  Measured on
+// a B200, us (5-point 2000^2 | 27-point 120^3 | power law 300,000 | power law 4M
+// rows | 512 banded matrices):
+//   contracted FP32, 7: 64 | 132 | 39.7 | 430 | 497   8: 64 | 132 | 40.0 | 404 | 462
+//   contracted FP64, 7: 97 | 279 | 53.4 | 481 | 573   8: 98 | 282 | 58.5 | 520 | 542
+//   bit-exact FP32,  6: 152 | 202 | 53.0 | 433        7: 134 | 179 | 52.7 | 403
+//   bit-exact FP64,  6: 171 | 244 | 84.7 | 537 | 632  7: 152 | 230 | 88.8 | 529 | 600
+// so 8 for contracted FP32 and batches, 7 for contracted FP64 and bit-exact FP32
+// and batches; bit-exact FP64 takes 7 where a warp has many tiles and 6 where
+// it has few (kManyTiles), where its share of L1 counts more.
+constexpr int kMinCtas = 6;
+constexpr int64_t kManyTiles = 16;  // tiles per warp at kMinCtas
+template <typename T, bool EXACT, bool MANY>
+__host__ __device__ constexpr int min_ctas() {
+  return EXACT ? (sizeof(T) == 4 || MANY ? 7 : kMinCtas) : (sizeof(T) == 4 || MANY ? 8 : 7);
+}
 
 // Row split (BACKEND_DEFAULT): a tile whose last row runs more than
 // `split_min` positions past the tile's window does not walk that tail
@@ -604,8 +615,8 @@ __device__ __forceinline__ void seg_tile(SegSmem<T, EXACT>& w, int lane, const i
 }
 
 template <typename T, bool EXACT, bool STANDARD, bool UNIT, bool SPLIT = false, bool V32 = false,
-          int RPL = 1>
-__global__ void __launch_bounds__(kThreads, EXACT ? kMinCtasExact : kMinCtasFast)
+          int RPL = 1, bool MANY = false>
+__global__ void __launch_bounds__(kThreads, (min_ctas<T, EXACT, MANY>()))
 seg_kernel(const int64_t* __restrict__ ptr, const int64_t* __restrict__ idx,
            const T* __restrict__ val, const T* __restrict__ x, int64_t incx, T* __restrict__ y,
            int64_t incy, T alpha, T beta, const int64_t* __restrict__ tile_row, int64_t ntiles,
@@ -789,13 +800,13 @@ __global__ void batch_bounds_kernel(const ascb_batch_item* __restrict__ items, i
 
 // (512 banded matrices of up to 16,384 rows, half bandwidth up to 31, FP64, B200:
 // 612 us on tiles of at most 32 rows with 16-byte loads and nothing asked for
-// early, 572 us; bit-exact 707 and 630; half bandwidth up to 5 218 and 168.  The
-// DRAM floor of the first is 358 us: latency, 28 warps an SM at 72 registers.)
+// early, 542 us; bit-exact 707 and 600.  The DRAM floor of the first is 358 us:
+// latency, 32 warps an SM.)
 // Warps take `chunk` consecutive tiles at a time.  What a tile needs is asked for
 // a step early: the next ticket while the current tiles run, the next tile's
 // bounds and row offsets (same matrix) while the current tile runs.
 template <typename T, bool EXACT, bool UNIT, bool V32>
-__global__ void __launch_bounds__(kThreads, EXACT ? kMinCtasExact : kMinCtasFast)
+__global__ void __launch_bounds__(kThreads, (min_ctas<T, EXACT, true>()))
 seg_batch_kernel(const ascb_batch_item* __restrict__ items, int64_t count,
                  const int64_t* __restrict__ bounds, int64_t total_tiles,
                  unsigned long long* __restrict__ queue, int chunk, T alpha, T beta) {
@@ -887,13 +898,13 @@ inline bool aligned32(const ascb_csr* a) {
   return ((reinterpret_cast<uintptr_t>(a->idx) | reinterpret_cast<uintptr_t>(a->val)) & 31u) == 0;
 }
 
-template <typename T, bool EXACT, bool STANDARD, bool UNIT, bool V32, int RPL>
+template <typename T, bool EXACT, bool STANDARD, bool UNIT, bool V32, int RPL, bool MANY>
 int launch_v(cudaStream_t stream, const ascb_csr* a, T alpha, T beta, const ascb_vec* x,
              const ascb_vec* y, const int64_t* tile_row, int64_t ntiles, int sm_count) {
-  auto kernel = seg_kernel<T, EXACT, STANDARD, UNIT, false, V32, RPL>;
+  auto kernel = seg_kernel<T, EXACT, STANDARD, UNIT, false, V32, RPL, MANY>;
   const int64_t ctas_needed = (ntiles + kWarpsPerCta - 1) / kWarpsPerCta;  // a tile a warp
   const int64_t resident_ctas = static_cast<int64_t>(sm_count > 0 ? sm_count : 148) *
-                                resident<T, EXACT, STANDARD, UNIT, (V32 ? 4 : 0) + 16 * RPL>(kernel);
+                                resident<T, EXACT, STANDARD, UNIT, (V32 ? 4 : 0) + 16 * RPL + (MANY ? 256 : 0)>(kernel);
   const unsigned blocks = static_cast<unsigned>(
       ctas_needed < 1 ? 1 : (ctas_needed < resident_ctas ? ctas_needed : resident_ctas));
   kernel<<<blocks, kThreads, 0, stream>>>(
@@ -906,11 +917,19 @@ int launch_v(cudaStream_t stream, const ascb_csr* a, T alpha, T beta, const ascb
 template <typename T, bool EXACT, bool STANDARD, bool UNIT, int RPL>
 int launch(cudaStream_t stream, const ascb_csr* a, T alpha, T beta, const ascb_vec* x,
            const ascb_vec* y, const int64_t* tile_row, int64_t ntiles, int sm_count) {
-  return aligned32(a)
-             ? launch_v<T, EXACT, STANDARD, UNIT, true, RPL>(stream, a, alpha, beta, x, y,
-                                                            tile_row, ntiles, sm_count)
-             : launch_v<T, EXACT, STANDARD, UNIT, false, RPL>(stream, a, alpha, beta, x, y,
-                                                             tile_row, ntiles, sm_count);
+  const bool wide = aligned32(a);
+  if constexpr (EXACT && sizeof(T) == 8) {
+    if (ntiles > kManyTiles * ascb_seg_one_pass_tiles(sm_count)) {
+      return wide ? launch_v<T, EXACT, STANDARD, UNIT, true, RPL, true>(stream, a, alpha, beta, x,
+                                                                       y, tile_row, ntiles, sm_count)
+                  : launch_v<T, EXACT, STANDARD, UNIT, false, RPL, true>(
+                        stream, a, alpha, beta, x, y, tile_row, ntiles, sm_count);
+    }
+  }
+  return wide ? launch_v<T, EXACT, STANDARD, UNIT, true, RPL, false>(stream, a, alpha, beta, x, y,
+                                                                    tile_row, ntiles, sm_count)
+              : launch_v<T, EXACT, STANDARD, UNIT, false, RPL, false>(stream, a, alpha, beta, x, y,
+                                                                     tile_row, ntiles, sm_count);
 }
 
 template <typename T, bool STANDARD, bool UNIT, bool V32, int RPL>
@@ -1030,7 +1049,7 @@ extern "C" int ascb_spmv_seg_alignment(void) { return 16; }
 // FP64, bit-exact, B200: 20.6 us with a partition and four tiles to a warp,
 // 8.3 us (DRAM floor 1.7).
 extern "C" int64_t ascb_seg_one_pass_tiles(int sm_count) {
-  return static_cast<int64_t>(sm_count > 0 ? sm_count : 148) * ascb::kMinCtasExact *
+  return static_cast<int64_t>(sm_count > 0 ? sm_count : 148) * ascb::kMinCtas *
          ascb::kWarpsPerCta;
 }
 

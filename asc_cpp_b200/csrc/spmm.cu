@@ -320,7 +320,7 @@ __device__ __forceinline__ void long_row_exact(const RowArgs<T>& a, int64_t o, i
 }
 
 template <typename T, int N, int G, int J, bool EXACT, bool WHOLE>
-__global__ void __launch_bounds__(kThreads, J * N * sizeof(T) > 16 ? 4 : 5) spmm_rows_kernel(RowArgs<T> a) {
+__global__ void __launch_bounds__(kThreads, J * N * sizeof(T) > 16 || J == 4 ? 4 : 5) spmm_rows_kernel(RowArgs<T> a) {
   constexpr int kGroups = kThreads / G;
   __shared__ __align__(16) unsigned char buffer[long_bytes<T, N, G, J, EXACT>()];
   __shared__ int long_rows[kLongRows];  // (round, group) they came up in
@@ -530,7 +530,11 @@ int64_t long_row_limit(const ascb_csr* a) {
 
 template <typename T, int N, int G, int J>
 int launch_rows(cudaStream_t s, bool exact, bool whole, const RowArgs<T>& a, int sm) {
-  const unsigned grid = grid_for(a.rows, kThreads / G, sm);
+  // Two wide chunks a lane run with the 4 CTAs per SM that are resident: more
+  // consecutive rows share an L1 at a time.  Against 8 per SM (k = 128, FP32,
+  // exact): 27-point 96^3 713 / 748 us, 5-point 700^2 167 / 173; a power law,
+  // whose uneven rows want the smaller shares, 846 / 766.
+  const unsigned grid = grid_for(a.rows, kThreads / G, J * N * sizeof(T) > 16 ? (sm + 1) / 2 : sm);
   if (exact) {
     if (whole) {
       spmm_rows_kernel<T, N, G, J, true, true><<<grid, kThreads, 0, s>>>(a);
@@ -551,22 +555,28 @@ int launch_rows(cudaStream_t s, bool exact, bool whole, const RowArgs<T>& a, int
 // per warp); wider rows take two chunks per lane (more independent loads in
 // flight, and a CTA covers more consecutive rows whose right-hand-side rows
 // then hit in L1).  Single elements: up to four per lane, so that k = 128
-// reads a row's entries once.
+// reads a row's entries once.  More than 32 chunks of 16 bytes take a warp per
+// row where rows average 12 or more entries (`wide`), half a warp in passes
+// where they are shorter: power law (16 a row), k = 200, FP32 exact 1156
+// against 1513 us, contracted 781 / 961; 27-point 64^3, k = 128, FP64 396 / 467
+// and 413 / 453; 5-point 500^2, k = 100, FP64 158 / 147 and 203 / 168.  Single
+// elements for the exact form at 32 or more chunks, as was, took 3476 us on the
+// 16 x 16 blocks (k = 128, FP32; 2141) and 1104 on the power law (k = 64, FP64;
+// 794).
 template <typename T, int N>
-int launch_by_width(cudaStream_t s, bool exact, bool whole, const RowArgs<T>& a, int sm) {
+int launch_by_width(cudaStream_t s, bool exact, bool whole, bool wide, const RowArgs<T>& a,
+                    int sm) {
 #define ASCB_ROWS(G, J) return launch_rows<T, N, G, J>(s, exact, whole, a, sm)
   if (a.chunks <= 1) ASCB_ROWS(1, 1);
   if (a.chunks <= 2) ASCB_ROWS(2, 1);
   if (a.chunks <= 4) ASCB_ROWS(2, 2);
   if (a.chunks <= 8) ASCB_ROWS(4, 2);
   if (a.chunks <= 16) ASCB_ROWS(8, 2);
-  if constexpr (N * sizeof(T) < 16) {
-    if (a.chunks > 32) {
-      if constexpr (N == 1) {
-        if (a.chunks > 64) ASCB_ROWS(32, 4);
-      }
-      ASCB_ROWS(32, 2);
+  if (a.chunks > 32 && (N * sizeof(T) < 16 || wide)) {
+    if constexpr (N == 1) {
+      if (a.chunks > 64) ASCB_ROWS(32, 4);
     }
+    ASCB_ROWS(32, 2);
   }
   ASCB_ROWS(16, 2);
 #undef ASCB_ROWS
@@ -586,19 +596,14 @@ int spmm_rows(cudaStream_t s, bool exact, const ascb_csr* m, int64_t k, const vo
   };
   int n = kMost;
   while (n > 1 && !divides(n, width, ldb, b)) n /= 2;
-  bool whole = c_layout == ASCB_ROW_MAJOR && divides(n, k, ldc, c);
-  // the exact form at 32 or more 16-byte chunks per row runs faster on single
-  // elements (measured on both matrices above)
-  if (exact && n == kMost && width / n >= 32) {
-    n = 1;
-    whole = c_layout == ASCB_ROW_MAJOR;
-  }
+  const bool whole = c_layout == ASCB_ROW_MAJOR && divides(n, k, ldc, c);
+  const bool wide = m->nnz >= 12 * m->rows;
   a.chunks = width / n;
   if (n == 4) {
-    if constexpr (sizeof(T) == 4) return launch_by_width<T, 4>(s, exact, whole, a, sm);
+    if constexpr (sizeof(T) == 4) return launch_by_width<T, 4>(s, exact, whole, wide, a, sm);
   }
-  if (n == 2) return launch_by_width<T, 2>(s, exact, whole, a, sm);
-  return launch_by_width<T, 1>(s, exact, whole, a, sm);
+  if (n == 2) return launch_by_width<T, 2>(s, exact, whole, wide, a, sm);
+  return launch_by_width<T, 1>(s, exact, whole, wide, a, sm);
 }
 
 // Rows past four times the mean and 32 go to the whole block: a warp takes as

@@ -66,7 +66,9 @@ constexpr int kMaxDevices = 64;
 //   bit-exact FP64,  6: 171 | 244 | 84.7 | 537 | 632  7: 152 | 230 | 88.8 | 529 | 600
 // so 8 for contracted FP32 and batches, 7 for contracted FP64 and bit-exact FP32
 // and batches; bit-exact FP64 takes 7 where a warp has many tiles and 6 where
-// it has few (kManyTiles), where its share of L1 counts more.
+// it has few (kManyTiles), where its share of L1 counts more, or where alpha = 1
+// and beta = 0 (4M-row power law 515 us at 6, 547 at 7; with general factors 531
+// and 514).
 constexpr int kMinCtas = 6;
 constexpr int64_t kManyTiles = 16;  // tiles per warp at kMinCtas
 template <typename T, bool EXACT, bool MANY>
@@ -616,7 +618,8 @@ __device__ __forceinline__ void seg_tile(SegSmem<T, EXACT>& w, int lane, const i
 
 template <typename T, bool EXACT, bool STANDARD, bool UNIT, bool SPLIT = false, bool V32 = false,
           int RPL = 1, bool MANY = false>
-__global__ void __launch_bounds__(kThreads, (min_ctas<T, EXACT, MANY>()))
+__global__ void __launch_bounds__(kThreads,
+                                  (min_ctas<T, EXACT, MANY && !(EXACT && UNIT)>()))
 seg_kernel(const int64_t* __restrict__ ptr, const int64_t* __restrict__ idx,
            const T* __restrict__ val, const T* __restrict__ x, int64_t incx, T* __restrict__ y,
            int64_t incy, T alpha, T beta, const int64_t* __restrict__ tile_row, int64_t ntiles,

@@ -78,18 +78,18 @@ constexpr int kWarps = kThreads / 32;
 constexpr int64_t kLongRow = 64;
 // Entries of a row that are waited for together, and CTAs per SM the kernel is
 // compiled for.  Level order runs one CTA per SM and has registers to spare.
-// Row order needs rows in flight as much as it needs whole rows in a batch: 3
-// entries (4 CTAs) are best while a row has at most 4 (its diagonal included),
-// 2 entries (5 CTAs) beyond: lower triangle of a 1000^2 5-point Laplacian 3.2
-// against 5.8 ms, of a 100^3 27-point stencil 3.3 against 2.6 ms (FP64, B200;
-// one entry at a time 5.3 and 3.9 ms).
+// Row order needs rows in flight as much as it needs whole rows in a batch, and
+// runs 4 CTAs (64 registers): 3 entries are best while a row has at most 4 (its
+// diagonal included), 2 beyond.  Lower triangle of a 1000^2 5-point Laplacian,
+// 3 and 2 entries: 3.1 and 5.8 ms; of a 100^3 27-point stencil 3.3 and 2.3 (2.6
+// with 5 CTAs, whose registers spill), a 4M-row power law exact 8.0 and 7.3
+// (9.4), 2M random rows 454 and 381 (488) (FP64, B200; one entry at a time
+// 5.4, 4.0, 7.5 and 455).
 constexpr int kLevelBatch = 4;
 constexpr int kShortRow = 4;
 constexpr int kShortBatch = 3;
 constexpr int kLongBatch = 2;
-__host__ __device__ constexpr int trsv_ctas(bool levels, int batch) {
-  return levels ? 1 : (batch == kShortBatch ? 4 : 5);
-}
+__host__ __device__ constexpr int trsv_ctas(bool levels) { return levels ? 1 : 4; }
 constexpr uint64_t kWaitNs = 2000000000ull;
 constexpr uint32_t kMaxPolls = 1u << 26;
 
@@ -336,16 +336,25 @@ __device__ void warp_row(const ascb_trsv& a, int64_t row, T alpha, T* pub, Contr
   if (lane == 0) value = A::mul(alpha, x[elem(row, 0, a.ld, a.row_major != 0)]);
   T acc = A::zero();
   T diag = A::zero();
+  // indices and values are fetched one chunk ahead of the waits (4M-row power
+  // law in level order, exact 6.6 -> 5.6 ms, contracted 5.2 -> 4.3)
+  int64_t next_c = 0;
+  T next_v = A::zero();
+  auto fetch = [&](int64_t p) {
+    if (p >= end) return;
+    next_c = __ldg(a.idx + p);
+    next_v = A::load(val + p);
+  };
+  fetch(beg + lane);
   for (int64_t p0 = beg; p0 < end; p0 += 32) {
     const int64_t p = p0 + lane;
     bool dep = false;
     bool is_diag = false;
-    T v = A::zero();
+    const int64_t c = next_c;
+    const T v = a.conj ? A::conj(next_v) : next_v;
     T prod = A::zero();
+    fetch(p + 32);
     if (p < end) {
-      const int64_t c = __ldg(a.idx + p);
-      v = A::load(val + p);
-      if (a.conj) v = A::conj(v);
       is_diag = c == row;
       dep = !is_diag && !outside(a, c, row);
       if (dep) {
@@ -393,7 +402,7 @@ __device__ void warp_row(const ascb_trsv& a, int64_t row, T alpha, T* pub, Contr
 
 // One right-hand side; LEVELS: in the level order of an analysis.
 template <typename T, bool EXACT, bool LEVELS, int kBatch>
-__global__ void __launch_bounds__(kThreads, trsv_ctas(LEVELS, kBatch))
+__global__ void __launch_bounds__(kThreads, trsv_ctas(LEVELS))
 trsv_single(ascb_trsv a, T alpha) {
   using A = Ar<T>;
   __shared__ T solved_value[kWarps][32];

@@ -24,6 +24,7 @@
 //     scatter form for FAST transposed products without a plan.
 #include "common.cuh"
 #include "kernels.h"
+#include "round_part.h"
 
 namespace ascb {
 namespace {
@@ -156,10 +157,9 @@ complex_rows(const int64_t* __restrict__ ptr, const int64_t* __restrict__ idx,
       }
       if (w + kRound < end) entries(w + kRound);
       __syncwarp();
-      const int from = static_cast<int>((b > w ? b : w) - w);
-      const int64_t to = e - w < kRound ? e - w : kRound;
+      const RoundPart part = round_part(b, e, w, kRound);
 #pragma unroll 4
-      for (int q = from; q < to; ++q) s = cadd<EXACT>(s, prod[q]);
+      for (int q = part.from; q < part.to; ++q) s = cadd<EXACT>(s, prod[q]);
       __syncwarp();  // the products are replaced
     }
     if constexpr (!EXACT) join();

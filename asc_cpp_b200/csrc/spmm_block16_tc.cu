@@ -44,7 +44,7 @@
 // the epilogue of one overlaps the MMAs of the next.
 // Every wait is bounded: one that runs out records 1 in *status, tells the
 // other roles to stop (a shared flag), and the CTA waits (bounded) for its own
-// MMAs before it frees its tensor memory.
+// MMAs and copies before it frees its tensor memory.
 #include <cstddef>
 
 #include "common.cuh"
@@ -210,11 +210,14 @@ bt_tiles_kernel(const float* __restrict__ b, int64_t ldb, int64_t k, int64_t b_r
   }
 }
 
-// bounded wait for phase `parity` of `bar`; false if it ran out or another
-// role of the CTA gave up (*abort)
+// Bounded wait of a whole warp for phase `parity` of `bar`; false if it ran out
+// or another role of the CTA gave up (*abort).  Lanes leave the polls one by
+// one, so the warp votes: all of its lanes act on the same answer, and what
+// follows (elect.sync, tcgen05.ld, the commits of the MMAs' own thread) finds
+// it converged.
 __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, const int* abort) {
-  for (uint32_t i = 0; i < kWaitLimit; ++i) {
-    uint32_t ok;
+  uint32_t ok = 0;
+  for (uint32_t i = 0; i < kWaitLimit && ok == 0; ++i) {
     asm volatile(
         "{\n .reg .pred p;\n"
         " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
@@ -222,10 +225,9 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, const i
         : "=r"(ok)
         : "r"(smem_u32(bar)), "r"(parity), "r"(kSuspendNs)
         : "memory");
-    if (ok) return true;
-    if (abort != nullptr && *reinterpret_cast<const volatile int*>(abort)) return false;
+    if (ok == 0 && abort != nullptr && *reinterpret_cast<const volatile int*>(abort)) break;
   }
-  return false;
+  return __all_sync(0xffffffffu, ok != 0) != 0;
 }
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&d)[16]) {
@@ -241,7 +243,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&d)[16]) {
 
 // Roles: warps 0..3 produce (warp p stages the blocks whose running index is
 // p mod 4, in stage p, and runs the epilogue for TMEM lanes 32p..32p+31);
-// warp 4 follows the same sequence and its lane 0 issues the MMAs.
+// warp 4 follows the same sequence and an elected lane issues the MMAs.
 // Barriers: full[p] (32 producer lanes arrive) -> MMAs -> empty[p]
 // (tcgen05.commit); at the end of a block row the
 // MMA thread commits dfull[a] for accumulator a, the producers read D and
@@ -367,8 +369,11 @@ block16_tc_kernel(const int64_t* __restrict__ ptr, const int64_t* __restrict__ i
       }
       ++itm;
     }
+    // giving up: this warp's last copy must not arrive after the CTA is gone
+    // (all lanes of the warp have arrived, so the phase ends with the copy)
+    if (failed && uses > 0) wait_bar(&s.full[p], (uses - 1) & 1u, nullptr);
   } else {
-    // ---------------- MMA issuer (warp 4: every lane waits, lane 0 issues) ----
+    // ---------------- MMA issuer (warp 4: every lane waits, one issues) ----
     uint32_t it = 0, itm = 0;
     for (int64_t item = blockIdx.x; item < items && !failed; item += gridDim.x) {
       const int64_t br = item / chunks;

@@ -78,13 +78,17 @@ constexpr int kWarps = kThreads / 32;
 constexpr int64_t kLongRow = 64;
 // Entries of a row that are waited for together, and CTAs per SM the kernel is
 // compiled for.  Level order runs one CTA per SM and has registers to spare.
-// Row order needs rows in flight as much as it needs whole rows in a batch, and
-// runs 4 CTAs (64 registers): 3 entries are best while a row has at most 4 (its
-// diagonal included), 2 beyond.  Lower triangle of a 1000^2 5-point Laplacian,
-// 3 and 2 entries: 3.1 and 5.8 ms; of a 100^3 27-point stencil 3.3 and 2.3 (2.6
-// with 5 CTAs, whose registers spill), a 4M-row power law exact 8.0 and 7.3
-// (9.4), 2M random rows 454 and 381 (488) (FP64, B200; one entry at a time
-// 5.4, 4.0, 7.5 and 455).
+// Row order runs 4 CTAs (64 registers; with 5 and more the polls of the rows in
+// flight get into each other's way: 5-point triangle 3.1 -> 5.2 ms): 3 entries
+// while a row stores at most 4, 2 beyond.  Row order, exact FP64, B200, ms; the
+// columns: one entry at a time | 2 or 3 together, every batch waiting for its round
+// of polls | batches without a dependency passed over (now):
+//   triangles: 5-point 1000^2 5.41 | 3.13 | 3.05, 9-point 700^2 4.72 | 4.44 | 3.25,
+//     7-point 100^3 1.62 | 2.31 | 1.50, 27-point 60^3 1.85 | 0.96 | 0.90,
+//     bidiagonal 100,000 73 | 30 | 29, random, 5 a row, 1M rows 0.060 | 0.067 | 0.063
+//   the same matrices stored whole: 7.08 | 8.52 | 4.55, 6.45 | 8.51 | 4.52,
+//     2.25 | 3.09 | 2.11, 2.73 | 3.72 | 2.07, 84 | 30 | 29, 0.072 | 0.084 | 0.072
+// With 3 entries together beyond 4: 9-point triangle 4.7, 27-point 1.4.
 constexpr int kLevelBatch = 4;
 constexpr int kShortRow = 4;
 constexpr int kShortBatch = 3;
@@ -506,14 +510,26 @@ trsv_single(ascb_trsv a, T alpha) {
           if (need == 0u) {
             p += kBatch;
             progressed = true;
-            if (p < end) {
-              open_batch();
-            } else {
+            auto finish = [&]() {
               if (!a.unit) value = A::div(value, diag);
               solved_value[warp][lane] = value;
               x[elem(row, 0, a.ld, row_major)] = value;
               A::publish(pub + row, value);
               done = true;
+            };
+            // a lane that is through goes ahead of those that fetch (rows of few entries;
+            // beyond, rows that never wait are 3 to 10% faster the other way round)
+            constexpr bool kFinishFirst = !LEVELS && kBatch == kShortBatch;
+            if (kFinishFirst && p >= end) {
+              finish();
+            } else {
+              if (p < end) {
+                open_batch();
+                // batches without a dependency (the diagonal, the other triangle of a
+                // matrix stored whole) must not cost a round of polls each
+                while (!LEVELS && need == 0u && (p += kBatch) < end) open_batch();
+              }
+              if (p >= end) finish();
             }
           }
         }

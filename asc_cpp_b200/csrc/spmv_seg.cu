@@ -63,17 +63,17 @@ constexpr int kMaxDevices = 64;
 //   contracted FP32, 7: 64 | 132 | 39.7 | 430 | 497   8: 64 | 132 | 40.0 | 404 | 462
 //   contracted FP64, 7: 97 | 279 | 53.4 | 481 | 573   8: 98 | 282 | 58.5 | 520 | 542
 //   bit-exact FP32,  6: 152 | 202 | 53.0 | 433        7: 134 | 179 | 52.7 | 403
-//   bit-exact FP64,  6: 171 | 244 | 84.7 | 537 | 632  7: 152 | 230 | 88.8 | 529 | 600
-// so 8 for contracted FP32 and batches, 7 for contracted FP64 and bit-exact FP32
-// and batches; bit-exact FP64 takes 7 where a warp has many tiles and 6 where
-// it has few (kManyTiles), where its share of L1 counts more, or where alpha = 1
-// and beta = 0 (4M-row power law 515 us at 6, 547 at 7; with general factors 531
-// and 514).
+//   bit-exact FP64,  6: 172 | 245 | 89.5 | 544 | 632  7: 153 | 231 | 93.2 | 574 | 600
+// so 8 for contracted FP32 and batches, 7 for contracted FP64, bit-exact FP32 and
+// bit-exact batches, 6 for bit-exact FP64.  The last depends on the matrix: at 7
+// the products staged in shared memory leave too little L1 for columns spread at
+// random over the whole width (power laws), and nothing the host knows tells
+// those from the grids; a power law whose rows spread their columns evenly takes
+// 546 at 6 and 528 at 7.  alpha and beta make no difference to it.
 constexpr int kMinCtas = 6;
-constexpr int64_t kManyTiles = 16;  // tiles per warp at kMinCtas
-template <typename T, bool EXACT, bool MANY>
+template <typename T, bool EXACT, bool BATCH>
 __host__ __device__ constexpr int min_ctas() {
-  return EXACT ? (sizeof(T) == 4 || MANY ? 7 : kMinCtas) : (sizeof(T) == 4 || MANY ? 8 : 7);
+  return EXACT ? (sizeof(T) == 4 || BATCH ? 7 : kMinCtas) : (sizeof(T) == 4 || BATCH ? 8 : 7);
 }
 
 // Row split (BACKEND_DEFAULT): a tile whose last row runs more than
@@ -617,9 +617,8 @@ __device__ __forceinline__ void seg_tile(SegSmem<T, EXACT>& w, int lane, const i
 }
 
 template <typename T, bool EXACT, bool STANDARD, bool UNIT, bool SPLIT = false, bool V32 = false,
-          int RPL = 1, bool MANY = false>
-__global__ void __launch_bounds__(kThreads,
-                                  (min_ctas<T, EXACT, MANY && !(EXACT && UNIT)>()))
+          int RPL = 1>
+__global__ void __launch_bounds__(kThreads, (min_ctas<T, EXACT, false>()))
 seg_kernel(const int64_t* __restrict__ ptr, const int64_t* __restrict__ idx,
            const T* __restrict__ val, const T* __restrict__ x, int64_t incx, T* __restrict__ y,
            int64_t incy, T alpha, T beta, const int64_t* __restrict__ tile_row, int64_t ntiles,
@@ -901,13 +900,13 @@ inline bool aligned32(const ascb_csr* a) {
   return ((reinterpret_cast<uintptr_t>(a->idx) | reinterpret_cast<uintptr_t>(a->val)) & 31u) == 0;
 }
 
-template <typename T, bool EXACT, bool STANDARD, bool UNIT, bool V32, int RPL, bool MANY>
+template <typename T, bool EXACT, bool STANDARD, bool UNIT, bool V32, int RPL>
 int launch_v(cudaStream_t stream, const ascb_csr* a, T alpha, T beta, const ascb_vec* x,
              const ascb_vec* y, const int64_t* tile_row, int64_t ntiles, int sm_count) {
-  auto kernel = seg_kernel<T, EXACT, STANDARD, UNIT, false, V32, RPL, MANY>;
+  auto kernel = seg_kernel<T, EXACT, STANDARD, UNIT, false, V32, RPL>;
   const int64_t ctas_needed = (ntiles + kWarpsPerCta - 1) / kWarpsPerCta;  // a tile a warp
   const int64_t resident_ctas = static_cast<int64_t>(sm_count > 0 ? sm_count : 148) *
-                                resident<T, EXACT, STANDARD, UNIT, (V32 ? 4 : 0) + 16 * RPL + (MANY ? 256 : 0)>(kernel);
+                                resident<T, EXACT, STANDARD, UNIT, (V32 ? 4 : 0) + 16 * RPL>(kernel);
   const unsigned blocks = static_cast<unsigned>(
       ctas_needed < 1 ? 1 : (ctas_needed < resident_ctas ? ctas_needed : resident_ctas));
   kernel<<<blocks, kThreads, 0, stream>>>(
@@ -920,19 +919,11 @@ int launch_v(cudaStream_t stream, const ascb_csr* a, T alpha, T beta, const ascb
 template <typename T, bool EXACT, bool STANDARD, bool UNIT, int RPL>
 int launch(cudaStream_t stream, const ascb_csr* a, T alpha, T beta, const ascb_vec* x,
            const ascb_vec* y, const int64_t* tile_row, int64_t ntiles, int sm_count) {
-  const bool wide = aligned32(a);
-  if constexpr (EXACT && sizeof(T) == 8) {
-    if (ntiles > kManyTiles * ascb_seg_one_pass_tiles(sm_count)) {
-      return wide ? launch_v<T, EXACT, STANDARD, UNIT, true, RPL, true>(stream, a, alpha, beta, x,
-                                                                       y, tile_row, ntiles, sm_count)
-                  : launch_v<T, EXACT, STANDARD, UNIT, false, RPL, true>(
-                        stream, a, alpha, beta, x, y, tile_row, ntiles, sm_count);
-    }
-  }
-  return wide ? launch_v<T, EXACT, STANDARD, UNIT, true, RPL, false>(stream, a, alpha, beta, x, y,
-                                                                    tile_row, ntiles, sm_count)
-              : launch_v<T, EXACT, STANDARD, UNIT, false, RPL, false>(stream, a, alpha, beta, x, y,
-                                                                     tile_row, ntiles, sm_count);
+  return aligned32(a)
+             ? launch_v<T, EXACT, STANDARD, UNIT, true, RPL>(stream, a, alpha, beta, x, y,
+                                                            tile_row, ntiles, sm_count)
+             : launch_v<T, EXACT, STANDARD, UNIT, false, RPL>(stream, a, alpha, beta, x, y,
+                                                             tile_row, ntiles, sm_count);
 }
 
 template <typename T, bool STANDARD, bool UNIT, bool V32, int RPL>

@@ -45,11 +45,13 @@ struct asc_sb_batch {
   std::int64_t total_tiles = 0;
   std::int64_t total_bounds = 0;
   int chunk = 4;
+  bool chunk_set = false;  // by the caller or a tuning run: taken as it is
   int ctas_per_sm = 0;
   // captured graph and the launch it holds
   cudaGraphExec_t exec = nullptr;
   double g_alpha = 0.0, g_beta = 0.0;
   int g_chunk = 0, g_ctas = 0, g_exact = -1;
+  bool g_chunk_set = false;
 };
 
 namespace {
@@ -152,8 +154,8 @@ int EnqueuePersistent(cudaStream_t stream, const asc_sb_batch& b, int exact, dou
   if (e != cudaSuccess) return static_cast<int>(e);
   return ascb_spmv_seg_batch(stream, Dtype(b.element_kind), exact, b.unit ? 1 : 0,
                              b.wide ? 1 : 0, b.items_dev,
-                             b.count, b.bounds, b.total_tiles, b.queue, b.chunk, b.ctas_per_sm,
-                             alpha, beta, sm_count);
+                             b.count, b.bounds, b.total_tiles, b.queue, b.chunk,
+                             b.chunk_set ? 0 : 1, b.ctas_per_sm, alpha, beta, sm_count);
 }
 
 void DropGraph(asc_sb_batch* b) {
@@ -195,7 +197,8 @@ Status RunBatch(const ContextView& v, asc_sb_batch* b, double alpha, double beta
   if (!b->aligned) return PerMatrix(v, *b, exact, alpha, beta);
   if (b->total_tiles == 0) return Status::Ok();
   if (b->exec != nullptr && b->g_alpha == alpha && b->g_beta == beta && b->g_exact == exact &&
-      b->g_chunk == b->chunk && b->g_ctas == b->ctas_per_sm) {
+      b->g_chunk == b->chunk && b->g_chunk_set == b->chunk_set &&
+      b->g_ctas == b->ctas_per_sm) {
     return Enqueued(v, static_cast<int>(cudaGraphLaunch(b->exec, v.stream)),
                     "CUDA could not launch the batch graph");
   }
@@ -380,6 +383,7 @@ int asc_sb_batch_set_schedule(asc_sb_context* context, asc_sb_batch* batch, int3
     return Done(v, Fail(ASC_SB_INVALID_ARGUMENT, "batch schedule is out of range"));
   }
   batch->chunk = chunk_tiles;
+  batch->chunk_set = true;
   batch->ctas_per_sm = ctas_per_sm;
   return Done(v, Status::Ok());
 }
@@ -460,6 +464,7 @@ int asc_sb_batch_capture(asc_sb_context* context, asc_sb_batch* batch, double al
   batch->g_beta = beta;
   batch->g_exact = exact;
   batch->g_chunk = batch->chunk;
+  batch->g_chunk_set = batch->chunk_set;
   batch->g_ctas = batch->ctas_per_sm;
   return Done(v, Status::Ok());
 }
@@ -487,6 +492,8 @@ int asc_sb_batch_autotune(asc_sb_context* context, asc_sb_batch* batch, double a
   if (e == cudaSuccess) e = cudaEventCreate(&stop);
   float best = -1.0f;
   int best_chunk = batch->chunk, best_ctas = batch->ctas_per_sm;
+  const bool was_set = batch->chunk_set;
+  batch->chunk_set = true;
   for (int chunk : kChunks) {
     for (int ctas : kCtas) {
       if (e != cudaSuccess) break;
@@ -513,6 +520,7 @@ int asc_sb_batch_autotune(asc_sb_context* context, asc_sb_batch* batch, double a
   if (start != nullptr) (void)cudaEventDestroy(start);
   if (stop != nullptr) (void)cudaEventDestroy(stop);
   batch->chunk = best_chunk;
+  batch->chunk_set = best >= 0.0f || was_set;
   batch->ctas_per_sm = best_ctas;
   if (e != cudaSuccess) {
     (void)cudaStreamSynchronize(v.stream);

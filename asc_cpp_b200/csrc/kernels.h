@@ -143,12 +143,12 @@ int ascb_batch_tile_bounds(void* stream, const ascb_batch_item* items, int64_t c
                            int64_t* bounds, int64_t total_bounds, int64_t items_per_tile,
                            int64_t weight, int sm_count);
 // Persistent work-queue SpMV over all tiles of the batch: warps take `chunk`
-// tiles at a time from *queue (zero before the launch); ctas_per_sm = 0 uses
-// the occupancy limit.  The tiles are the segmented kernel's own.  Index and
+// tiles at a time (fit = 1: fewer where some resident warp would get none) from
+// *queue (zero before the launch); ctas_per_sm = 0 uses the occupancy limit.  The tiles are the segmented kernel's own.  Index and
 // value arrays must be 16-byte aligned (wide = 1: all of them 32-byte aligned).
 int ascb_spmv_seg_batch(void* stream, int dtype, int exact, int unit, int wide,
                         const ascb_batch_item* items, int64_t count, const int64_t* bounds,
-                        int64_t total_tiles, unsigned long long* queue, int chunk,
+                        int64_t total_tiles, unsigned long long* queue, int chunk, int fit,
                         int ctas_per_sm, double alpha, double beta, int sm_count);
 
 // ---- learned variant selector (features + MLP cost model) ----

@@ -1136,14 +1136,14 @@ namespace {
 template <typename T, bool EXACT, bool UNIT, bool V32>
 int launch_batch(cudaStream_t s, const ascb_batch_item* items, int64_t count,
                  const int64_t* bounds, int64_t total_tiles, unsigned long long* queue, int chunk,
-                 int ctas_per_sm, T alpha, T beta, int sm) {
+                 int fit, int ctas_per_sm, T alpha, T beta, int sm) {
   auto kernel = seg_batch_kernel<T, EXACT, UNIT, V32>;
   int per_sm = ctas_per_sm;
   if (per_sm <= 0) per_sm = resident<T, EXACT, false, UNIT, V32 ? 7 : 1>(kernel);
   const int64_t cap = static_cast<int64_t>(sm > 0 ? sm : 148) * per_sm;
   // no more tiles at a time than leave every resident warp some
   const int64_t share = (total_tiles + cap * kWarpsPerCta - 1) / (cap * kWarpsPerCta);
-  if (chunk > share) chunk = static_cast<int>(share);
+  if (fit && chunk > share) chunk = static_cast<int>(share);
   const int64_t warps_needed = (total_tiles + chunk - 1) / chunk;
   const int64_t ctas_needed = (warps_needed + kWarpsPerCta - 1) / kWarpsPerCta;
   const unsigned blocks =
@@ -1155,11 +1155,12 @@ int launch_batch(cudaStream_t s, const ascb_batch_item* items, int64_t count,
 template <typename T>
 int batch_typed(cudaStream_t s, int exact, int unit, int wide, const ascb_batch_item* items,
                 int64_t count, const int64_t* bounds, int64_t total_tiles,
-                unsigned long long* queue, int chunk, int ctas, double alpha, double beta, int sm) {
+                unsigned long long* queue, int chunk, int fit, int ctas, double alpha, double beta,
+                int sm) {
   const T a = static_cast<T>(alpha), b = static_cast<T>(beta);
 #define ASCB_BATCH(E, U, V)                                                                     \
-  return launch_batch<T, E, U, V>(s, items, count, bounds, total_tiles, queue, chunk, ctas, a, \
-                                  b, sm)
+  return launch_batch<T, E, U, V>(s, items, count, bounds, total_tiles, queue, chunk, fit,     \
+                                  ctas, a, b, sm)
   if (exact) {
     if (unit && wide) ASCB_BATCH(true, true, true);
     if (unit) ASCB_BATCH(true, true, false);
@@ -1193,15 +1194,15 @@ extern "C" int ascb_batch_tile_bounds(void* stream, const ascb_batch_item* items
 extern "C" int ascb_spmv_seg_batch(void* stream, int dtype, int exact, int unit, int wide,
                                    const ascb_batch_item* items, int64_t count,
                                    const int64_t* bounds, int64_t total_tiles,
-                                   unsigned long long* queue, int chunk, int ctas_per_sm,
+                                   unsigned long long* queue, int chunk, int fit, int ctas_per_sm,
                                    double alpha, double beta, int sm_count) {
   if (count <= 0 || total_tiles <= 0) return 0;
   if (chunk < 1) chunk = 1;
   auto s = static_cast<cudaStream_t>(stream);
   if (dtype == ASCB_F64) {
     return ascb::batch_typed<double>(s, exact, unit, wide, items, count, bounds, total_tiles, queue,
-                                     chunk, ctas_per_sm, alpha, beta, sm_count);
+                                     chunk, fit, ctas_per_sm, alpha, beta, sm_count);
   }
   return ascb::batch_typed<float>(s, exact, unit, wide, items, count, bounds, total_tiles, queue,
-                                  chunk, ctas_per_sm, alpha, beta, sm_count);
+                                  chunk, fit, ctas_per_sm, alpha, beta, sm_count);
 }

@@ -627,7 +627,9 @@ ASC_SB_API int asc_sb_batch_create(asc_sb_context* context, int64_t count,
                                    asc_sb_batch** out);
 ASC_SB_API int asc_sb_batch_destroy(asc_sb_batch* batch);
 /* Schedule of the persistent launch: tiles a warp takes per queue grab
- * (1..4096) and CTAs per SM (0 = the occupancy limit, else 1..32). */
+ * (1..4096) and CTAs per SM (0 = the occupancy limit, else 1..32).  Until one
+ * is set or tuned, the tiles read 4 and are fewer where a batch is so small
+ * that some of the warps would get none. */
 ASC_SB_API int asc_sb_batch_set_schedule(asc_sb_context* context,
                                          asc_sb_batch* batch,
                                          int32_t chunk_tiles,

@@ -89,7 +89,13 @@ struct RowArgs {
   int64_t long_row;  // rows with more entries are set aside
 };
 
-constexpr int kLongRows = 64;  // rows a block can set aside (more: taken where they stand)
+constexpr int kLongRows = 64;  // rows a block can list
+// Entries per group up to which one warp takes a listed row, contracted form of up
+// to 4 lanes a row: 8 rows go side by side without a barrier, a longer one keeps
+// its warp too long.
+// 1M-row power law, FP32, k = 1 / 16, us: 16 entries 144 / 400, 32 141 / 379, 64
+// 143 / 376, 256 152 / 409.
+constexpr int kWarpShare = 32;
 
 // Shared memory comes out of L1, which serves B to neighbouring rows (10 KB a
 // block cost the 27-point stencil 9% at k = 128), so long rows get little of
@@ -195,15 +201,15 @@ __device__ __forceinline__ void store_c(const RowArgs<T>& a, int64_t o, int64_t 
   }
 }
 
-// A row set aside, by the whole block, contracted: every group sums a share
+// A row set aside, contracted: every group of the block (or warp) sums a share
 // of the entries, shuffles join the groups of a warp, and the warps add to one
 // sum in shared memory in turn.
-template <typename T, int N, int G, int J, bool WHOLE, bool COLUMNS = false>
+template <typename T, int N, int G, int J, bool WHOLE, bool COLUMNS = false, bool BLOCK = true>
 __device__ __forceinline__ void long_row_fast(const RowArgs<T>& a, int64_t o, int64_t pb,
                                               int64_t pe, T* smem) {
-  constexpr int kGroups = kThreads / G;
+  constexpr int kGroups = (BLOCK ? kThreads : 32) / G;
   const int lane = threadIdx.x % G;
-  const int group = threadIdx.x / G;
+  const int group = threadIdx.x / G % kGroups;
   const int64_t share = (pe - pb + kGroups - 1) / kGroups;
   const int64_t q0 = pb + group * share < pe ? pb + group * share : pe;
   const int64_t q1 = q0 + share < pe ? q0 + share : pe;
@@ -225,6 +231,20 @@ __device__ __forceinline__ void long_row_fast(const RowArgs<T>& a, int64_t o, in
 #pragma unroll
         for (int m = G; m < 32; m <<= 1) acc[t][e] += shfl_xor(acc[t][e], m);
       }
+    }
+    if constexpr (!BLOCK) {
+      if (threadIdx.x % 32 < G) {
+#pragma unroll
+        for (int t = 0; t < J; ++t) {
+          if (!live[t]) continue;
+          T old[N];
+          load_c<T, N, WHOLE>(a, o, v0 + t * G + lane, old);
+#pragma unroll
+          for (int e = 0; e < N; ++e) acc[t][e] = fma(a.alpha, acc[t][e], old[e]);
+          store_c<T, N, WHOLE>(a, o, v0 + t * G + lane, acc[t]);
+        }
+      }
+      continue;
     }
     for (int w = 0; w < kThreads / 32; ++w) {
       if (static_cast<int>(threadIdx.x) / 32 == w && threadIdx.x % 32 < G) {
@@ -319,8 +339,12 @@ __device__ __forceinline__ void long_row_exact(const RowArgs<T>& a, int64_t o, i
   }
 }
 
+// CTAs per SM: at 5 the contracted narrow forms spill (27-point 64^3, FP64, k = 2
+// 55 us, 36 at 4; 100,000 random rows of 64 entries want the warps: FP32, k = 8
+// 79 us, 95 at 4).
 template <typename T, int N, int G, int J, bool EXACT, bool WHOLE>
-__global__ void __launch_bounds__(kThreads, J * N * sizeof(T) > 16 || J == 4 ? 4 : 5) spmm_rows_kernel(RowArgs<T> a) {
+__global__ void __launch_bounds__(kThreads, J * N * sizeof(T) > 16 || J == 4 || !EXACT ? 4 : 5)
+spmm_rows_kernel(RowArgs<T> a) {
   constexpr int kGroups = kThreads / G;
   __shared__ __align__(16) unsigned char buffer[long_bytes<T, N, G, J, EXACT>()];
   __shared__ int long_rows[kLongRows];  // (round, group) they came up in
@@ -342,10 +366,11 @@ __global__ void __launch_bounds__(kThreads, J * N * sizeof(T) > 16 || J == 4 ? 4
                                << (threadIdx.x % 32 / G * G);
         at = __shfl_sync(group, at, 0, G);
       }
-      if (at < kLongRows) {
-        if (lane == 0) long_rows[at] = static_cast<int>((o - first) / step * kGroups + threadIdx.x / G);
-        continue;
+      if (lane == 0 && at < kLongRows) {
+        long_rows[at] = static_cast<int>((o - first) / step * kGroups + threadIdx.x / G);
       }
+      // (stored order gives the same bits whoever adds)
+      if (!EXACT || at < kLongRows) continue;
     }
     for (int64_t v0 = 0; v0 < a.chunks; v0 += int64_t{G} * J) {
       // C is read first where that costs few registers: one wait less at the end
@@ -377,16 +402,83 @@ __global__ void __launch_bounds__(kThreads, J * N * sizeof(T) > 16 || J == 4 ? 4
     }
   }
   __syncthreads();
-  const int count = long_count < kLongRows ? long_count : kLongRows;
-  for (int i = 0; i < count; ++i) {
-    const int64_t o = static_cast<int64_t>(blockIdx.x) * kGroups + long_rows[i] % kGroups +
-                      long_rows[i] / kGroups * step;
-    const int64_t pb = __ldg(a.ptr + o);
-    const int64_t pe = __ldg(a.ptr + o + 1);
-    if constexpr (EXACT) {
-      long_row_exact<T, N, G, J>(a, o, pb, pe, reinterpret_cast<T*>(buffer));
-    } else {
-      long_row_fast<T, N, G, J, WHOLE>(a, o, pb, pe, reinterpret_cast<T*>(buffer));
+  auto row_at = [&](int place) {
+    return static_cast<int64_t>(blockIdx.x) * kGroups + place % kGroups + place / kGroups * step;
+  };
+  if constexpr (EXACT) {
+    const int count = long_count < kLongRows ? long_count : kLongRows;
+    for (int i = 0; i < count; ++i) {
+      const int64_t o = row_at(long_rows[i]);
+      long_row_exact<T, N, G, J>(a, o, __ldg(a.ptr + o), __ldg(a.ptr + o + 1),
+                                 reinterpret_cast<T*>(buffer));
+    }
+    return;
+  }
+  // Contracted: who takes a row follows from its length and from how many there
+  // are, never from the order in which they were listed, so that it is added up
+  // the same way on every run.
+  int count = long_count;
+  if (count == 0) return;
+  const bool listed = count <= kLongRows;
+  const int places = listed ? count : static_cast<int>((a.rows + step - 1) / step) * kGroups;
+  // rows of a range of places with more than `least` entries into the list
+  auto list_again = [&](int begin, int end, int64_t least) {
+    __syncthreads();
+    if (threadIdx.x == 0) long_count = 0;
+    __syncthreads();
+    for (int i = begin + static_cast<int>(threadIdx.x); i < end; i += kThreads) {
+      const int64_t o = row_at(i);
+      if (o < a.rows && __ldg(a.ptr + o + 1) - __ldg(a.ptr + o) > least) {
+        const int at = atomicAdd(&long_count, 1);
+        if (at < kLongRows) long_rows[at] = i;
+      }
+    }
+    __syncthreads();
+    count = long_count;
+  };
+  if constexpr (G <= 4) {
+    // rows of up to `most` entries to a warp each, the others to the whole block;
+    // where there are too many of those for the list, `most` grows until they fit
+    int64_t most = kWarpShare * (32 / G);
+    while (!listed) {
+      list_again(0, places, max(most, a.long_row));
+      if (count <= kLongRows) break;
+      most *= 4;
+    }
+    for (int i = threadIdx.x / 32; i < places; i += kThreads) {
+      auto row_of = [&](int lane_of) {
+        const int j = i + lane_of * (kThreads / 32);
+        return j < places ? row_at(listed ? long_rows[j] : j) : a.rows;
+      };
+      unsigned mine;
+      {
+        const int64_t o = row_of(threadIdx.x % 32);
+        const int64_t n = o < a.rows ? __ldg(a.ptr + o + 1) - __ldg(a.ptr + o) : 0;
+        mine = __ballot_sync(0xffffffffu, n > a.long_row && n <= most);
+      }
+      for (; mine != 0u; mine &= mine - 1u) {
+        const int64_t o = row_of(__ffs(mine) - 1);
+        long_row_fast<T, N, G, J, WHOLE, false, false>(a, o, __ldg(a.ptr + o),
+                                                       __ldg(a.ptr + o + 1), nullptr);
+      }
+    }
+    for (int i = 0; i < count; ++i) {
+      const int64_t o = row_at(long_rows[i]);
+      const int64_t pb = __ldg(a.ptr + o);
+      const int64_t pe = __ldg(a.ptr + o + 1);
+      if (pe - pb > most) {
+        long_row_fast<T, N, G, J, WHOLE>(a, o, pb, pe, reinterpret_cast<T*>(buffer));
+      }
+    }
+  } else {
+    // all to the whole block, as many places at a time as the list holds
+    for (int begin = 0; begin < places; begin += kLongRows) {
+      if (!listed) list_again(begin, min(begin + kLongRows, places), a.long_row);
+      for (int i = 0; i < count; ++i) {
+        const int64_t o = row_at(long_rows[i]);
+        long_row_fast<T, N, G, J, WHOLE>(a, o, __ldg(a.ptr + o), __ldg(a.ptr + o + 1),
+                                         reinterpret_cast<T*>(buffer));
+      }
     }
   }
 }

@@ -655,10 +655,18 @@ int launch_rows(cudaStream_t s, bool exact, bool whole, const RowArgs<T>& a, int
 // elements for the exact form at 32 or more chunks, as was, took 3476 us on the
 // 16 x 16 blocks (k = 128, FP32; 2141) and 1104 on the power law (k = 64, FP64;
 // 794).
+//
+// Few long rows (`few`: 32 or more entries on average, and one lane a row makes at
+// most two CTAs per SM) spread over four lanes whatever the width, even if some
+// stay idle: an SM more is worth more than a lane.  Rows of 64 entries, FP32,
+// k = 1 / 3, us, one and two lanes / four: 2,000 rows 20.6 / 10.3 and 14.4 / 10.3,
+// 40,000 rows 40.5 / 36.3 and 39.1 / 32.9, 100,000 rows 60 / 77 and 78 / 83; 8,192 rows
+// of 160 47 / 19 and 29 / 21; a power law of 5,000 rows with 16 entries on average 12.4 / 18.5.
 template <typename T, int N>
-int launch_by_width(cudaStream_t s, bool exact, bool whole, bool wide, const RowArgs<T>& a,
-                    int sm) {
+int launch_by_width(cudaStream_t s, bool exact, bool whole, bool wide, bool few,
+                    const RowArgs<T>& a, int sm) {
 #define ASCB_ROWS(G, J) return launch_rows<T, N, G, J>(s, exact, whole, a, sm)
+  if (few && a.chunks <= 4) ASCB_ROWS(4, 1);
   if (a.chunks <= 1) ASCB_ROWS(1, 1);
   if (a.chunks <= 2) ASCB_ROWS(2, 1);
   if (a.chunks <= 4) ASCB_ROWS(2, 2);
@@ -690,12 +698,13 @@ int spmm_rows(cudaStream_t s, bool exact, const ascb_csr* m, int64_t k, const vo
   while (n > 1 && !divides(n, width, ldb, b)) n /= 2;
   const bool whole = c_layout == ASCB_ROW_MAJOR && divides(n, k, ldc, c);
   const bool wide = m->nnz >= 12 * m->rows;
+  const bool few = m->nnz >= 32 * m->rows && m->rows <= int64_t{2} * (sm > 0 ? sm : 148) * kThreads;
   a.chunks = width / n;
   if (n == 4) {
-    if constexpr (sizeof(T) == 4) return launch_by_width<T, 4>(s, exact, whole, wide, a, sm);
+    if constexpr (sizeof(T) == 4) return launch_by_width<T, 4>(s, exact, whole, wide, few, a, sm);
   }
-  if (n == 2) return launch_by_width<T, 2>(s, exact, whole, wide, a, sm);
-  return launch_by_width<T, 1>(s, exact, whole, wide, a, sm);
+  if (n == 2) return launch_by_width<T, 2>(s, exact, whole, wide, few, a, sm);
+  return launch_by_width<T, 1>(s, exact, whole, wide, few, a, sm);
 }
 
 // Rows past four times the mean and 32 go to the whole block: a warp takes as

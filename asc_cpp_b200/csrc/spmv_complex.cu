@@ -13,8 +13,8 @@
 //     to 32 consecutive rows, whose entries lie one behind the other: all lanes
 //     form 128 products at a time in shared memory while the next 128 entries
 //     are on their way, and each row's lane adds its own in stored order (EXACT
-//     to y, FAST to a sum that y gets once, rounds inside one row by a warp
-//     tree).  With a warp per row and the products
+//     to y, FAST to a sum that y gets once, lanes to spare sharing a row and
+//     rounds inside one row by warp trees).  With a warp per row and the products
 //     handed to one sum by shuffles, rows of 27 entries left lanes idle and
 //     cost 4 x 27 dependent steps: 27-point stencil on 63^3, Z, bit-exact, B200:
 //     167 us, now 47 (DRAM floor 26).
@@ -84,7 +84,8 @@ template <typename R, bool EXACT, bool CONJ, bool UNIT, bool PAIR>
 __global__ void __launch_bounds__(kThreads)
 complex_rows(const int64_t* __restrict__ ptr, const int64_t* __restrict__ idx,
              const Cx<R>* __restrict__ val, const Cx<R>* __restrict__ x, int64_t incx,
-             Cx<R>* __restrict__ y, int64_t incy, Cx<R> alpha, int64_t rows, int per_warp) {
+             Cx<R>* __restrict__ y, int64_t incy, Cx<R> alpha, int64_t rows, int per_warp,
+             int log_share) {
   __shared__ Cx<R> staged[kThreads / 32][kRound];
   Cx<R>* prod = staged[threadIdx.x / 32];
   const int lane = threadIdx.x & 31;
@@ -93,7 +94,8 @@ complex_rows(const int64_t* __restrict__ ptr, const int64_t* __restrict__ idx,
                     per_warp;
        r0 < rows; r0 += warps * per_warp) {
     const int64_t last = r0 + per_warp < rows ? r0 + per_warp : rows;
-    const int64_t r = r0 + lane;
+    const int share = EXACT ? 1 : 1 << log_share;  // lanes of a row
+    const int64_t r = r0 + (EXACT ? lane : lane >> log_share);
     const bool mine = r < last;
     const int64_t end = __ldg(ptr + last);
     const int64_t b = mine ? __ldg(ptr + r) : end;
@@ -158,12 +160,22 @@ complex_rows(const int64_t* __restrict__ ptr, const int64_t* __restrict__ idx,
       if (w + kRound < end) entries(w + kRound);
       __syncwarp();
       const RoundPart part = round_part(b, e, w, kRound);
-#pragma unroll 4
-      for (int q = part.from; q < part.to; ++q) s = cadd<EXACT>(s, prod[q]);
+      // (loads 16 at a time ahead of the chain of sums; 4 at a time, power law of 262,144
+      // rows, bit-exact, C / Z: 87 / 139 us against 77 / 105)
+#pragma unroll 16
+      for (int q = part.from + (lane & (share - 1)); q < part.to; q += share) {
+        s = cadd<EXACT>(s, prod[q]);
+      }
       __syncwarp();  // the products are replaced
     }
-    if constexpr (!EXACT) join();
-    if (b < e) {  // (without entries y keeps its bits)
+    if constexpr (!EXACT) {
+      join();
+      for (int m = share >> 1; m > 0; m >>= 1) {
+        s.re += __shfl_xor_sync(0xffffffffu, s.re, m);
+        s.im += __shfl_xor_sync(0xffffffffu, s.im, m);
+      }
+    }
+    if (b < e && (lane & (share - 1)) == 0) {  // (without entries y keeps its bits)
       Cx<R>* yp = &at<UNIT>(y, r, incy);
       *yp = EXACT ? s : cadd<false>(*yp, s);
     }
@@ -274,13 +286,17 @@ int spmv_typed(cudaStream_t s, int mode, const ascb_csr* a, Cx<R> alpha, const a
   if (per_warp * mean > 4 * kRound) per_warp = 4 * kRound / mean;
   if (per_warp * mean > kRound && per_warp * mean < 2 * kRound) per_warp = kRound / mean;
   per_warp = per_warp < 1 ? 1 : (per_warp > 32 ? 32 : per_warp);
+  // FAST: the lanes that this leaves over share the rows (100,000 rows of 64 entries,
+  // one lane each / 4, C and Z, us: 52 / 38 and 69 / 51)
+  int log_share = 0;
+  while ((per_warp << (log_share + 1)) <= 32) ++log_share;
   const unsigned blocks = Blocks((a->rows + per_warp - 1) / per_warp * 32, sm);
   auto kernel = mode == 1 ? (pair ? complex_rows<R, true, CONJ, UNIT, true>
                                   : complex_rows<R, true, CONJ, UNIT, false>)
                           : (pair ? complex_rows<R, false, CONJ, UNIT, true>
                                   : complex_rows<R, false, CONJ, UNIT, false>);
   kernel<<<blocks, kThreads, 0, s>>>(ptr, idx, val, xd, x->stride, yd, y->stride, alpha, a->rows,
-                                     static_cast<int>(per_warp));
+                                     static_cast<int>(per_warp), log_share);
   return static_cast<int>(cudaGetLastError());
 }
 

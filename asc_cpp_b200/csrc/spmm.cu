@@ -72,11 +72,11 @@ struct Chunk<double, 2> {
   __device__ static double2 join(const double (&e)[2]) { return make_double2(e[0], e[1]); }
 };
 
-// One product C += alpha * A * B over contiguous rows of B.
+// One product C += alpha * A * B.
 template <typename T>
 struct RowArgs {
   int64_t rows;
-  int64_t k;       // columns of C; the last chunk of a packed B row may pass it
+  int64_t k;       // columns of C
   int64_t chunks;  // chunks of a row of B
   const int64_t* ptr;
   const int64_t* idx;
@@ -682,24 +682,24 @@ int launch_by_width(cudaStream_t s, bool exact, bool whole, bool wide, bool few,
 #undef ASCB_ROWS
 }
 
-// B in rows of `width` >= k elements (width > k: packed, zeros past k).
+// Row-major B.
 template <typename T>
 int spmm_rows(cudaStream_t s, bool exact, const ascb_csr* m, int64_t k, const void* b,
-              int64_t width, int64_t ldb, void* c, int c_layout, int64_t ldc, T alpha, int sm) {
+              int64_t ldb, void* c, int c_layout, int64_t ldc, T alpha, int sm) {
   constexpr int kMost = 16 / sizeof(T);
   RowArgs<T> a{m->rows, k, 0, m->ptr, m->idx, static_cast<const T*>(m->val),
                static_cast<const T*>(b), ldb, static_cast<T*>(c), 1, 1, alpha, long_row_limit(m)};
   (c_layout == ASCB_ROW_MAJOR ? a.c_row : a.c_col) = ldc;
-  auto divides = [](int64_t n, int64_t w, int64_t ld, const void* p) {
-    return w % n == 0 && ld % n == 0 &&
+  auto divides = [k](int64_t n, int64_t ld, const void* p) {
+    return k % n == 0 && ld % n == 0 &&
            (reinterpret_cast<uintptr_t>(p) & (static_cast<uintptr_t>(n) * sizeof(T) - 1)) == 0;
   };
   int n = kMost;
-  while (n > 1 && !divides(n, width, ldb, b)) n /= 2;
-  const bool whole = c_layout == ASCB_ROW_MAJOR && divides(n, k, ldc, c);
+  while (n > 1 && !divides(n, ldb, b)) n /= 2;
+  const bool whole = c_layout == ASCB_ROW_MAJOR && divides(n, ldc, c);
   const bool wide = m->nnz >= 12 * m->rows;
   const bool few = m->nnz >= 32 * m->rows && m->rows <= int64_t{2} * (sm > 0 ? sm : 148) * kThreads;
-  a.chunks = width / n;
+  a.chunks = k / n;
   if (n == 4) {
     if constexpr (sizeof(T) == 4) return launch_by_width<T, 4>(s, exact, whole, wide, few, a, sm);
   }
@@ -762,7 +762,7 @@ int spmm_typed(cudaStream_t s, int transpose, int exact, const ascb_csr* a, int6
     return static_cast<int>(cudaGetLastError());
   }
   if (b_layout == ASCB_ROW_MAJOR) {
-    return spmm_rows<T>(s, exact != 0, a, k, b, k, ldb, c, c_layout, ldc, alpha, sm);
+    return spmm_rows<T>(s, exact != 0, a, k, b, ldb, c, c_layout, ldc, alpha, sm);
   }
   return spmm_columns<T>(s, exact != 0, a, k, b, ldb, c, c_layout, ldc, alpha, sm);
 }

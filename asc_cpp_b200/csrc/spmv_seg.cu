@@ -121,10 +121,6 @@ __device__ __forceinline__ T product(T alpha, T v, T xv) {
   if (EXACT && STANDARD) return mul_rn(mul_rn(alpha, v), xv);
   return EXACT ? mul_rn(v, xv) : v * xv;
 }
-template <bool EXACT, typename T>
-__device__ __forceinline__ T add(T a, T b) {
-  return EXACT ? add_rn(a, b) : a + b;
-}
 template <bool EXACT, bool STANDARD, typename T>
 __device__ __forceinline__ T row_init(T y_old) {
   return (EXACT && STANDARD) ? y_old : T(0);
@@ -432,7 +428,7 @@ __device__ __forceinline__ void seg_tile(SegSmem<T, EXACT>& w, int lane, const i
     if (nonempty) w.rowid[ne_before + __popc(ne_mask & lt_mask)] = static_cast<int16_t>(k);
     if (mine && !nonempty && !STANDARD) {  // empty row: y = alpha*(+0) + beta*y
       T* yp = &at<UNIT>(y, r0 + k, incy);
-      *yp = finish<EXACT, STANDARD>(T(0), alpha, beta, yp);
+      *yp = finish<false, STANDARD>(T(0), alpha, beta, yp);
     }
     ne_before += __popc(ne_mask);
   }
@@ -445,7 +441,7 @@ __device__ __forceinline__ void seg_tile(SegSmem<T, EXACT>& w, int lane, const i
   const int vhi = lim - p0 < 0 ? 0 : (lim - p0 > kPer ? kPer : lim - p0);
   const uint32_t vmask = ((1u << vhi) - 1u) & ~((1u << vlo) - 1u);
   T p[kPer];
-  lane_products<T, EXACT, STANDARD, UNIT, V32>(p, vmask, idx + (a0 + p0), val + (a0 + p0), x, incx,
+  lane_products<T, false, STANDARD, UNIT, V32>(p, vmask, idx + (a0 + p0), val + (a0 + p0), x, incx,
                                           alpha);
   const uint32_t word = w.bits[lane >> 2];
   const uint32_t flags = (word >> ((lane & 3) * 8)) & 0xffu;
@@ -469,7 +465,6 @@ __device__ __forceinline__ void seg_tile(SegSmem<T, EXACT>& w, int lane, const i
   bool first_seg = true;  // still in the segment open at the lane's start
   T first_val = T(0);
   int first_rank = -1;
-  int first_end = kPer;   // position where the continued segment closes
 #pragma unroll
   for (int i = 0; i < kPer; ++i) {
     if ((flags >> i) & 1u) {
@@ -477,71 +472,42 @@ __device__ __forceinline__ void seg_tile(SegSmem<T, EXACT>& w, int lane, const i
         if (first_seg) {
           first_val = acc;
           first_rank = rank;
-          first_end = i;
         } else {
           T* yp = &at<UNIT>(y, r0 + w.rowid[rank - 1], incy);
-          *yp = finish<EXACT, STANDARD>(acc, alpha, beta, yp);
+          *yp = finish<false, STANDARD>(acc, alpha, beta, yp);
         }
       }
       first_seg = false;
       ++rank;
       acc = p[i];
-    } else if (!(EXACT && first_seg)) {
-      acc = add<EXACT>(acc, p[i]);
+    } else {
+      acc += p[i];
     }
   }
   const bool has_start = flags != 0u;
-  T c;  // this lane's carry out: the running sum of the row open at its end
-  T carry_in = T(0);
-  if (!EXACT) {
-    // segmented scan of the open tails: c = has_start ? acc : c_prev + acc
-    c = acc;
-    bool f = has_start;
+  // segmented scan of the open tails: c = has_start ? acc : c_prev + acc, the
+  // running sum of the row open at the lane's end
+  T c = acc;
+  bool f = has_start;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const T cu = __shfl_up_sync(0xffffffffu, c, o);
-      const bool fu = __shfl_up_sync(0xffffffffu, f, o);
-      if (lane >= o) {
-        if (!f) c = cu + c;
-        f = f || fu;
-      }
+  for (int o = 1; o < 32; o <<= 1) {
+    const T cu = __shfl_up_sync(0xffffffffu, c, o);
+    const bool fu = __shfl_up_sync(0xffffffffu, f, o);
+    if (lane >= o) {
+      if (!f) c = cu + c;
+      f = f || fu;
     }
-    carry_in = __shfl_up_sync(0xffffffffu, c, 1);
-    if (lane == 0) carry_in = T(0);
-    if (first_rank > 0) {  // continued row closed inside this lane
-      T* yp = &at<UNIT>(y, r0 + w.rowid[first_rank - 1], incy);
-      *yp = finish<EXACT, STANDARD>(carry_in + first_val, alpha, beta, yp);
-    }
-  } else {
-    // exact: the running sum is handed lane to lane; a lane whose first
-    // valid position starts a row (or that has no data) needs nothing.
-    bool resolved = !has_data || ((flags >> vlo) & 1u);
-    c = acc;
-    for (int step = 0; step < 32; ++step) {
-      const T cu = __shfl_up_sync(0xffffffffu, c, 1);
-      const bool ru = __shfl_up_sync(0xffffffffu, resolved, 1);
-      if (!resolved && ru) {
-        T s = cu;
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-          if (k >= vlo && k < first_end) s = add_rn(s, p[k]);
-        }
-        if (first_rank > 0) {
-          T* yp = &at<UNIT>(y, r0 + w.rowid[first_rank - 1], incy);
-          *yp = finish<EXACT, STANDARD>(s, alpha, beta, yp);
-          c = acc;
-        } else {
-          c = s;
-        }
-        resolved = true;
-      }
-      if (__all_sync(0xffffffffu, resolved)) break;
-    }
+  }
+  T carry_in = __shfl_up_sync(0xffffffffu, c, 1);
+  if (lane == 0) carry_in = T(0);
+  if (first_rank > 0) {  // continued row closed inside this lane
+    T* yp = &at<UNIT>(y, r0 + w.rowid[first_rank - 1], incy);
+    *yp = finish<false, STANDARD>(carry_in + first_val, alpha, beta, yp);
   }
   if (has_data && next_start && rank > 0 && p0 + kPer <= lim) {
     // the open segment closes at the lane end (row start or data end next)
     T* yp = &at<UNIT>(y, r0 + w.rowid[rank - 1], incy);
-    *yp = finish<EXACT, STANDARD>(c, alpha, beta, yp);
+    *yp = finish<false, STANDARD>(c, alpha, beta, yp);
   }
   const T carry_out = __shfl_sync(0xffffffffu, c, 31);
 
@@ -574,43 +540,23 @@ __device__ __forceinline__ void seg_tile(SegSmem<T, EXACT>& w, int lane, const i
     // long last row: the nonzeros past the window, 256 per round, each lane
     // 8 contiguous ones with vector loads (the window ends on an aligned
     // position: a0 + kItems, so every round starts aligned too)
-    T total;
     T part = T(0);
-    total = carry_out;
     for (int64_t q0 = base + window; q0 < base + span; q0 += kItems) {
       const int64_t rem = base + span - q0;
       const int cnt = static_cast<int>(rem < kItems ? rem : kItems);
       const int hi = cnt - p0 < 0 ? 0 : (cnt - p0 > kPer ? kPer : cnt - p0);
       const uint32_t m = (1u << hi) - 1u;
       T q[kPer];
-      lane_products<T, EXACT, STANDARD, UNIT, V32>(q, m, idx + (q0 + p0), val + (q0 + p0), x, incx,
+      lane_products<T, false, STANDARD, UNIT, V32>(q, m, idx + (q0 + p0), val + (q0 + p0), x, incx,
                                               alpha);
-      if (!EXACT) {
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) part += q[k];
-      } else {
-        // stored order: lane 0 adds the round's products from shared memory
-        store_run(w.prod + p0, lane, q);
-        __syncwarp();
-        if (lane == 0) {
-          int k = 0;
-          for (; k + 8 <= cnt; k += 8) {
-#pragma unroll
-            for (int u = 0; u < 8; ++u) total = add_rn(total, w.prod[k + u]);
-          }
-          for (; k < cnt; ++k) total = add_rn(total, w.prod[k]);
-        }
-        __syncwarp();
-      }
+      for (int k = 0; k < kPer; ++k) part += q[k];
     }
-    if (!EXACT) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) part += shfl_xor(part, o);
-      total = carry_out + part;
-    }
+    for (int o = 16; o > 0; o >>= 1) part += shfl_xor(part, o);
     if (lane == 0) {
       T* yp = &at<UNIT>(y, r0 + nr - 1, incy);
-      *yp = finish<EXACT, STANDARD>(total, alpha, beta, yp);
+      *yp = finish<false, STANDARD>(carry_out + part, alpha, beta, yp);
     }
   }
   __syncwarp();  // bitmap and row tables are rewritten by the next tile

@@ -12,12 +12,12 @@
 //
 // Rows far longer than the mean would each be one group's serial chain of
 // loads while the chip idles (a power-law matrix of 262,144 rows and 4.2 M
-// entries, FP32, B200: k = 50 950 us that way, 279 us with the rule below;
-// k = 8 968 and 79, k = 32 bit-exact 2240 and 211).
-// They are set aside and then taken by all groups of their block together:
-// FAST splits the entries and adds the groups' sums in a fixed order, EXACT
-// forms the products in parallel and adds them in stored order from shared
-// memory.
+// entries, FP32, B200: k = 50 950 us that way, 269 us with the rule below;
+// k = 8 968 and 68, k = 32 bit-exact 2240 and 211).
+// They are set aside and then taken by all groups of a warp or of their block
+// together: FAST splits the entries and adds the groups' sums in a fixed order,
+// EXACT (the block) forms the products in parallel and adds them in stored order
+// from shared memory.
 //
 // Column-major right-hand sides: a lane per row, several columns at a time
 // (spmm_columns_kernel), with the same rule for long rows.  One thread per
@@ -656,12 +656,14 @@ int launch_rows(cudaStream_t s, bool exact, bool whole, const RowArgs<T>& a, int
 // 16 x 16 blocks (k = 128, FP32; 2141) and 1104 on the power law (k = 64, FP64;
 // 794).
 //
-// Few long rows (`few`: 32 or more entries on average, and one lane a row makes at
-// most two CTAs per SM) spread over four lanes whatever the width, even if some
-// stay idle: an SM more is worth more than a lane.  Rows of 64 entries, FP32,
-// k = 1 / 3, us, one and two lanes / four: 2,000 rows 20.6 / 10.3 and 14.4 / 10.3,
-// 40,000 rows 40.5 / 36.3 and 39.1 / 32.9, 100,000 rows 60 / 77 and 78 / 83; 8,192 rows
-// of 160 47 / 19 and 29 / 21; a power law of 5,000 rows with 16 entries on average 12.4 / 18.5.
+// Few long rows (`few`: 32 or more entries on average, and four lanes a row make no
+// more CTAs than are resident) spread over four lanes whatever the width, even if
+// some stay idle: an SM more is worth more than a lane, a second wave is not.
+// FP32, k = 1 / 3, us, one and two lanes / four: 2,000 rows of 64 entries 20.6 / 10.3 and
+// 14.4 / 10.3, 37,800 rows 22.7 / 24.7 and 26.8 / 24.9; 8,192 rows of 160 47 / 19 and
+// 29 / 21, 24,576 rows of 496 128 / 101 and 132 / 104; in a second wave 49,152 rows of 976
+// bit-exact 451 / 457 and 351 / 469.  A power law of 5,000 rows, 16 entries on average,
+// 12.4 / 18.5.
 template <typename T, int N>
 int launch_by_width(cudaStream_t s, bool exact, bool whole, bool wide, bool few,
                     const RowArgs<T>& a, int sm) {
@@ -698,7 +700,8 @@ int spmm_rows(cudaStream_t s, bool exact, const ascb_csr* m, int64_t k, const vo
   while (n > 1 && !divides(n, ldb, b)) n /= 2;
   const bool whole = c_layout == ASCB_ROW_MAJOR && divides(n, ldc, c);
   const bool wide = m->nnz >= 12 * m->rows;
-  const bool few = m->nnz >= 32 * m->rows && m->rows <= int64_t{2} * (sm > 0 ? sm : 148) * kThreads;
+  const int64_t wave = (sm > 0 ? sm : 148) * (exact ? 5 : 4) * int64_t{kThreads / 4};  // rows
+  const bool few = m->nnz >= 32 * m->rows && m->rows <= wave;
   a.chunks = k / n;
   if (n == 4) {
     if constexpr (sizeof(T) == 4) return launch_by_width<T, 4>(s, exact, whole, wide, few, a, sm);

@@ -19,10 +19,11 @@ ROW = SparseBlasLayout.kRowMajor
 
 @pytest.mark.parametrize("dt", [np.float32, np.float64])
 @pytest.mark.parametrize("k", [1, 2, 3, 4, 6, 8, 12])
-@pytest.mark.parametrize("case", ["one", "few", "short", "edge", "past"])
+@pytest.mark.parametrize("case", ["one", "few", "short", "fast edge", "edge", "past"])
 def test_few_rows(cuda_lib, restatement, dt, k, case):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    rows = {"one": 1, "few": 1003, "short": 1003, "edge": 2 * sms * 256, "past": 2 * sms * 256 + 1}[case]
+    rows = {"one": 1, "few": 1003, "short": 1003, "fast edge": sms * 256,
+            "edge": sms * 320, "past": sms * 320 + 1}[case]
     if rows > 2000 and k not in (1, 3, 8):
         pytest.skip("the edge in rows at three widths")
     cols = 3000

@@ -17,7 +17,7 @@
 //     rounds inside one row by warp trees).  With a warp per row and the products
 //     handed to one sum by shuffles, rows of 27 entries left lanes idle and
 //     cost 4 x 27 dependent steps: 27-point stencil on 63^3, Z, bit-exact, B200:
-//     167 us, now 47 (DRAM floor 26).
+//     167 us, now 44 (DRAM floor 26).
 //   * scatter: FAST transposed products without a plan, one warp per stored
 //     row, atomic adds of both components.
 //   * SpMM: one thread per (row, right-hand side) in stored order, or the

@@ -276,7 +276,11 @@ ASC_SB_API int asc_sb_csr_spmv_no_alloc(asc_sb_context* context, double alpha,
  * (asc_sb_plan_create with ASC_SB_PLAN_TRANSPOSE), or, without a plan, one
  * rebuilt for the call in the context's scratch buffer (which grows, after a
  * stream drain, from the context's allocator).  BACKEND_DEFAULT without a
- * plan scatters with atomics. */
+ * plan scatters with atomics.
+ * DETERMINISTIC multiplies alpha into every entry, as the CPU template does.
+ * BACKEND_DEFAULT's real row products sum op(A) * x first and apply alpha once, for
+ * every layout and width: where that sum exceeds the element type's range, the
+ * result does too, however small alpha is. */
 ASC_SB_API int asc_sb_standard_spmv(asc_sb_context* context, int32_t op,
                                     double alpha_real, double alpha_imag,
                                     const asc_sb_sparse* matrix,

@@ -1,7 +1,7 @@
 """The SpMM row kernel where it can go wrong: rows far longer than the mean
-(taken by a whole block), chunk widths of 16, 8 and 4 bytes, every layout pair
-(column-major right-hand sides are packed into rows from about a million
-products on), and no scratch to pack into."""
+(taken by a warp or a whole block), chunk widths of 16, 8 and 4 bytes, every layout
+pair (column-major right-hand sides: the kernel with a lane per row), and a
+captured product."""
 
 import numpy as np
 import pytest

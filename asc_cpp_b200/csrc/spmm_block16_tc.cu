@@ -211,13 +211,15 @@ bt_tiles_kernel(const float* __restrict__ b, int64_t ldb, int64_t k, int64_t b_r
 }
 
 // Bounded wait of a whole warp for phase `parity` of `bar`; false if it ran out
-// or another role of the CTA gave up (*abort).  Lanes leave the polls one by
-// one, so the warp votes: all of its lanes act on the same answer, and what
-// follows (elect.sync, tcgen05.ld, the commits of the MMAs' own thread) finds
-// it converged.
+// or another role of the CTA gave up (*abort).  The warp votes on every poll: all
+// of its lanes leave together with the same answer, and what follows (elect.sync,
+// tcgen05.ld, the commits of the MMAs' own thread) finds it converged.  A lane whose
+// poll succeeded may poll again: the next phase needs this warp.  (Lanes that leave
+// one by one and vote once after the loop cost up to 7%: 65,536 rows, 2% dense
+// blocks, k = 8 / 32 / 128, B200, us: 306 / 344 / 413, this way 281 / 319 / 407.)
 __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, const int* abort) {
   uint32_t ok = 0;
-  for (uint32_t i = 0; i < kWaitLimit && ok == 0; ++i) {
+  for (uint32_t i = 0; i < kWaitLimit; ++i) {
     asm volatile(
         "{\n .reg .pred p;\n"
         " mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
@@ -225,7 +227,11 @@ __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, const i
         : "=r"(ok)
         : "r"(smem_u32(bar)), "r"(parity), "r"(kSuspendNs)
         : "memory");
-    if (ok == 0 && abort != nullptr && *reinterpret_cast<const volatile int*>(abort)) break;
+    if (__all_sync(0xffffffffu, ok != 0)) break;
+    if (abort != nullptr &&
+        __any_sync(0xffffffffu, *reinterpret_cast<const volatile int*>(abort))) {
+      break;
+    }
   }
   return __all_sync(0xffffffffu, ok != 0) != 0;
 }

@@ -1290,7 +1290,7 @@ Status StandardSpmm(asc_sb_context* ctx, const asc_sb_plan* plan, int op, double
     // dense 16 x 16 blocks: tensor cores (3xTF32), within the bound stated in
     // spmm_block16_tc.cu; faster than the CUDA-core kernels at every k
     // measured on B200 (65,536-row 2% block-sparse matrix, k = 8 / 32 / 128:
-    // 0.29 / 0.32 / 0.41 ms against 0.80 / 1.05 / 2.04 ms).  The B^T tile
+    // 0.28 / 0.32 / 0.41 ms against 0.79 / 1.06 / 2.22 ms).  The B^T tile
     // images of the call's pre-pass live in the context's scratch.
     unsigned char* tiles = nullptr;
     s = SolveScratch(ctx, RoundUp(ascb_block16_tiles_bytes(a.cols, c->columns), 256), &tiles);

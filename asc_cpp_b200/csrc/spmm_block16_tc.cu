@@ -493,8 +493,8 @@ extern "C" size_t ascb_block16_tiles_bytes(int64_t cols, int64_t k) {
          ascb::kTileFloats * sizeof(float);
 }
 
-// 65,536-row matrix with 2% dense blocks, B200, k = 8 / 32 / 128: 291 / 324 /
-// 410 us (six MMAs a block issued under `lane == 0`: 398 / 430 / 451); error
+// 65,536-row matrix with 2% dense blocks, B200, k = 8 / 32 / 128: 281 / 319 /
+// 407 us (six MMAs a block issued under `lane == 0`: 398 / 430 / 451); error
 // against 64 bits 3.4e-6 (1.0e-5).  At k = 128 the bound is the 16 KB of B images
 // a block brings from L2; below, the CTAs' MMA issue.  Feeding raw B through
 // registers into tensor memory as the MMA's A operand (8 KB a block, no
